@@ -293,7 +293,7 @@ typedef struct lgpu_stats {
      reference's object order (more than one mesh whose bounds contain the
      ray origin), re-traced with its linear object loop */
   uint64_t order_rays;
-  /* 1 if a traversal stack of the last render or trace grew past the 16
+  /* 1 if a traversal stack of the last render or trace grew past the
      entries per ray kept in shared memory into local memory */
   uint32_t local_stack;
   uint32_t reserved;

@@ -264,15 +264,9 @@ __global__ void __launch_bounds__(128, 10) wf_shade_adjoint(OneJob jobs, WaveSta
     if (live) {
       hero = in.hero[i];
       depth = in.depth[i];
-      HitRec h;
-      h.obj = __float_as_uint(w.hit[cap + i]);
-      if (h.obj != UINT32_MAX) {
-        h.z = w.hit[i];
-        h.face = __float_as_uint(w.hit[2 * cap + i]);
-        h.b0 = w.hit[3 * cap + i];
-        h.b1 = w.hit[4 * cap + i];
-        h.b2 = w.hit[5 * cap + i];
-        h.pl = f3{w.hit[6 * cap + i], w.hit[7 * cap + i], w.hit[8 * cap + i]};
+      uint32_t const obj = w.hobj[i];
+      if (obj != UINT32_MAX) {
+        HitRec const h = load_hit(w, i, obj);
         Ray const r = load_ray(in.ray, cap, i);
         HitInfo const H = finalize_hit(S, r, h);
         f3 const un = fnorm(r.u);

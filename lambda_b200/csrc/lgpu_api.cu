@@ -265,7 +265,9 @@ size_t wave_layout(uint8_t* base, uint32_t cap, uint32_t K, uint32_t npix, uint6
     pb->gw = adjoint ? c.take<float>(size_t(K) * n) : nullptr;
     pb->sidx = c.take<uint32_t>(n);
   }
-  ws.hit = c.take<float>(9 * n);
+  ws.hobj = c.take<uint32_t>(n);
+  ws.hita = c.take<float4>(n);
+  ws.hitb = c.take<float4>(n);
   ws.e_acc = c.take<float>(size_t(K) * n);
   ws.e_hero = c.take<float>(n);
   ws.e_item = c.take<uint32_t>(n);

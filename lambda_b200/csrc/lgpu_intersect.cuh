@@ -171,8 +171,12 @@ __device__ __forceinline__ float segment_box_entry(const float* bb, const Ray& r
   return tmin <= tmax ? tmin : kFltMax;
 }
 
+// the neighbours of a positive float
 __device__ __forceinline__ float prev_float(float z) {
   return __int_as_float(__float_as_int(z) - 1);
+}
+__device__ __forceinline__ float next_float(float z) {
+  return __int_as_float(__float_as_int(z) + 1);
 }
 
 // intersect::aabb_avx2 (cg.hpp:1295-1337) for child c of a wide node:

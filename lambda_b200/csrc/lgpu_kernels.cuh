@@ -59,7 +59,9 @@ struct WaveState {
   PathBuf in, out;     // current and next queue, swapped every iteration
   uint32_t* n_in;      // queue lengths (in ctl), swapped with the queues
   uint32_t* n_out;
-  float* hit;          // 9*cap closest hits of `in` (z, obj, face, b0, b1, b2, plx, ply, plz)
+  uint32_t* hobj;      // cap: object each path of `in` hit, UINT32_MAX: none
+  float4* hita;        // cap: the hit's face, b0, b1, b2 (written for hits only)
+  float4* hitb;        // cap: its local point and distance
   float* e_acc;        // K*cap: radiance of the paths ended this iteration
   float* e_hero;       // cap
   uint32_t* e_item;    // cap

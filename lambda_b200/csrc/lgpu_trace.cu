@@ -48,18 +48,10 @@ __global__ void __launch_bounds__(128) trace_store(DevScene S, WaveState w, uint
   uint32_t const i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
   uint32_t const cap = w.cap;
-  const float* hp = w.hit;
-  HitRec h;
-  h.z = hp[i];
-  h.obj = __float_as_uint(hp[cap + i]);
-  h.face = __float_as_uint(hp[2 * cap + i]);
-  h.b0 = hp[3 * cap + i];
-  h.b1 = hp[4 * cap + i];
-  h.b2 = hp[5 * cap + i];
-  h.pl = f3{hp[6 * cap + i], hp[7 * cap + i], hp[8 * cap + i]};
+  uint32_t const obj = w.hobj[i];
   lgpu_hit o;
-  if (h.obj != UINT32_MAX) {
-    HitInfo const H = finalize_hit(S, load_ray(w.in.ray, cap, i), h);
+  if (obj != UINT32_MAX) {
+    HitInfo const H = finalize_hit(S, load_ray(w.in.ray, cap, i), load_hit(w, i, obj));
     o.t = H.z;
     o.obj = H.obj;
     o.face = H.face;
@@ -69,7 +61,7 @@ __global__ void __launch_bounds__(128) trace_store(DevScene S, WaveState w, uint
     o.gn[0] = H.gn.x; o.gn[1] = H.gn.y; o.gn[2] = H.gn.z;
     o.front = H.front ? 1u : 0u;
   } else {
-    o.t = h.z;
+    o.t = kFltMax;
     o.obj = UINT32_MAX;
     o.face = UINT32_MAX;
     o.mat = UINT32_MAX;
@@ -123,7 +115,9 @@ size_t trace_wave_layout(uint8_t* base, uint32_t cap, WaveState& ws) {
   ws = WaveState{};
   ws.cap = cap;
   ws.in.ray = reinterpret_cast<float*>(take(6 * sizeof(float) * size_t(cap)));
-  ws.hit = reinterpret_cast<float*>(take(9 * sizeof(float) * size_t(cap)));
+  ws.hobj = reinterpret_cast<uint32_t*>(take(sizeof(uint32_t) * size_t(cap)));
+  ws.hita = reinterpret_cast<float4*>(take(sizeof(float4) * size_t(cap)));
+  ws.hitb = reinterpret_cast<float4*>(take(sizeof(float4) * size_t(cap)));
   ws.fb_queue = reinterpret_cast<uint32_t*>(take(sizeof(uint32_t) * size_t(cap)));
   ws.sray = reinterpret_cast<float*>(take(8 * sizeof(float) * size_t(cap)));
   ws.s_vis = take(size_t(cap));

@@ -1,14 +1,12 @@
-// lgpu_traverse.cuh — the instance-level traversal used by the wavefront
-// kernels: one loop over instance-BVH and mesh-BVH nodes with a single
-// stack, so that all lanes of a warp execute the same "pop, test, push"
-// step whatever level they are at.
+// lgpu_traverse.cuh — the instance-level traversals used by the wavefront
+// kernels, over one stack for instance-BVH and mesh-BVH nodes.
 //
-// Entering a mesh pushes a marker and the mesh root; popping the marker
-// returns to world space.  A leaf of the instance BVH is consumed one object
-// at a time (the rest of the leaf is pushed back), which visits objects and
-// mesh nodes in exactly the order of the nested traversal in
-// lgpu_intersect.cuh, so results are identical to it (and therefore to the
-// reference's intersect::scene, see scene_hit).
+// trace_tlas runs one ray to its end; an entered mesh is delimited on the
+// stack by a marker.  The persistent kernels run the same search as a state
+// machine (TraceState) whose node, leaf and object steps the lanes of a warp
+// take together.  Both visit objects and mesh nodes in the order of the
+// nested traversal in lgpu_intersect.cuh, so results are identical to it
+// (and therefore to the reference's intersect::scene, see scene_hit).
 //
 // The stack keeps its first kSmemStack entries in shared memory, laid out
 // entry-major (entry k of thread t at k*blockDim.x + t) so a warp's pushes
@@ -31,7 +29,10 @@ namespace lgpu {
 // node tests; the reference-order traversal keeps the exact test.
 constexpr float kTravSlack = 1.f + 1.f / 65536.f;
 
-constexpr int kSmemStack = 16;
+// 10 entries: the persistent kernels push at most two per node and seldom
+// need more, and the shared memory this leaves is L1 for the nodes (8 and 16
+// were 1 % slower on the benchmark frame)
+constexpr int kSmemStack = 10;
 constexpr int kLocalStack = kStackCap + kTlasStackCap + 4 - kSmemStack;
 constexpr uint32_t kMarker = 0xFFFFFFFEu;
 
@@ -40,15 +41,16 @@ struct SplitStack {
   uint32_t stride;
   StackEntry* lm;  // local overflow
   int sp;
-  // kTravLocalStack once an entry beyond the shared part was used (merged
-  // into the thread's TravStats::flags when its work is counted)
-  uint32_t spill;
+  // kTravLocalStack once an entry beyond the shared part was used, and
+  // kTravOverflow (merged into the thread's TravStats::flags when its work is
+  // counted)
+  uint32_t flags;
   // this thread's column of the world-ray save area (9 floats, stride 128;
-  // trace_step only)
+  // persistent kernels only)
   float* ws = nullptr;
   __device__ __forceinline__ StackEntry& at(int k) {
     if (k < kSmemStack) return sm[k * stride];
-    spill = kTravLocalStack;
+    flags |= kTravLocalStack;
     return lm[k - kSmemStack];
   }
   // push and pop branch to a shared or a local access: through at()'s
@@ -58,7 +60,7 @@ struct SplitStack {
     if (sp < kSmemStack) {
       sm[sp * stride] = e;
     } else {
-      spill = kTravLocalStack;
+      flags |= kTravLocalStack;
       lm[sp - kSmemStack] = e;
     }
     sp++;
@@ -281,149 +283,346 @@ __device__ __forceinline__ bool trace_tlas(const DevScene& S, const Ray& w, HitR
   return hit_any;
 }
 
-// trace_tlas as a resumable state machine: trace_begin sets up a ray,
-// trace_step processes one stack entry.  The persistent trace kernels call
-// trace_step in a loop shared by the whole warp and give a lane a new ray
-// as soon as its ray is finished, so lanes do not idle while the longest ray
-// of their warp completes.
-// Besides the ray, a query has a mode (`any`: stop at the first hit, as
-// shadow rays do), an object to skip and an index limit (objects with a
-// higher or equal index are ignored), and counts the meshes whose bounds
-// contain the ray origin (n_inside).
-// `w` is the ray of the current level: the world ray, or the mesh-local ray
-// while a mesh is entered, when the world ray waits in shared memory
-// (SplitStack::ws) until the mesh's end marker.  One ray in registers
-// instead of two lets the closest-hit kernel run 6 blocks per SM without
-// spills (traversal -4 % measured).
-struct TraceState {
-  Ray w;
-  f3 mr;
-  HitRec h;
-  uint32_t skip, ilimit, cur;
-  float zs, cur_exit;
-  uint32_t n_inside;
-  bool any, in_mesh, lowered, cur_inside, hit_any;
-};
+// ---- resumable traversal of the persistent kernels ---------------------------------
 
-__device__ __forceinline__ void trace_begin(const DevScene& S, TraceState& t, SplitStack& st) {
-  t.h.inside = false;
-  t.in_mesh = t.lowered = t.cur_inside = t.hit_any = false;
-  t.cur = 0;
-  t.n_inside = 0;
-  t.zs = t.cur_exit = 0.f;
-  st.sp = 0;
-  if (S.n_objects == 0) return;  // no instance BVH: every ray misses
-  float const t0 = segment_box_entry(S.tlas_bounds, t.w, t.h.z);
-  if (t0 != kFltMax) st.push(StackEntry{S.tlas_root, t0});
+// Two single-precision values in one 64-bit register pair: Blackwell's
+// packed add and multiply round each half as the scalar operation does, so
+// the planes of two boxes cost two issue slots instead of four.
+__device__ __forceinline__ uint64_t pack2(float x) {
+  uint64_t r;
+  asm("mov.b64 %0, {%1, %1};" : "=l"(r) : "f"(x));
+  return r;
+}
+__device__ __forceinline__ void unpack2(uint64_t v, float& a, float& b) {
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(v));
+}
+__device__ __forceinline__ uint64_t add2(uint64_t a, uint64_t b) {
+  uint64_t r;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+__device__ __forceinline__ uint64_t mul2(uint64_t a, uint64_t b) {
+  uint64_t r;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+__device__ __forceinline__ float max3(float a, float b, float c) {
+  float r;
+  asm("max.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
+  return r;
+}
+__device__ __forceinline__ float min3(float a, float b, float c) {
+  float r;
+  asm("min.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
+  return r;
 }
 
-// One step of trace_tlas; returns true when the ray is finished (stack
-// empty, or an any-hit query found a hit).  ANY fixes the mode at compile
-// time; otherwise t.any selects it.
+// Entry distances of all 8 child boxes (node_boxes_t's values, two children
+// per instruction), handed one by one to f(child, entry, hit).
+template <class F>
+__device__ __forceinline__ void node_children(const WideNode& nd, const Ray& r, float t_max, F f) {
+  bool const nx = r.inv.x < 0.f, ny = r.inv.y < 0.f, nz = r.inv.z < 0.f;
+  const ulonglong2* const nrx = reinterpret_cast<const ulonglong2*>(nx ? nd.hix : nd.lox);
+  const ulonglong2* const frx = reinterpret_cast<const ulonglong2*>(nx ? nd.lox : nd.hix);
+  const ulonglong2* const nry = reinterpret_cast<const ulonglong2*>(ny ? nd.hiy : nd.loy);
+  const ulonglong2* const fry = reinterpret_cast<const ulonglong2*>(ny ? nd.loy : nd.hiy);
+  const ulonglong2* const nrz = reinterpret_cast<const ulonglong2*>(nz ? nd.hiz : nd.loz);
+  const ulonglong2* const frz = reinterpret_cast<const ulonglong2*>(nz ? nd.loz : nd.hiz);
+  uint64_t const px = pack2(-r.p.x), py = pack2(-r.p.y), pz = pack2(-r.p.z);
+  uint64_t const ix = pack2(r.inv.x), iy = pack2(r.inv.y), iz = pack2(r.inv.z);
+  uint64_t const slack = pack2(kTravSlack);
+#pragma unroll
+  for (int h = 0; h < 2; h++) {
+    ulonglong2 const a = nrx[h], b = frx[h], c = nry[h], d = fry[h], e = nrz[h], g = frz[h];
+#pragma unroll
+    for (int k = 0; k < 2; k++) {
+      float x0, x1, y0, y1, z0, z1;
+      unpack2(mul2(add2(k ? a.y : a.x, px), ix), x0, x1);
+      unpack2(mul2(add2(k ? c.y : c.x, py), iy), y0, y1);
+      unpack2(mul2(add2(k ? e.y : e.x, pz), iz), z0, z1);
+      float const n0 = fmaxf(max3(x0, y0, z0), kBias), n1 = fmaxf(max3(x1, y1, z1), kBias);
+      unpack2(mul2(add2(k ? b.y : b.x, px), ix), x0, x1);
+      unpack2(mul2(add2(k ? d.y : d.x, py), iy), y0, y1);
+      unpack2(mul2(add2(k ? g.y : g.x, pz), iz), z0, z1);
+      float f0 = fminf(min3(x0, y0, z0), t_max), f1 = fminf(min3(x1, y1, z1), t_max);
+      uint64_t ff;
+      asm("mov.b64 %0, {%1, %2};" : "=l"(ff) : "f"(f0), "f"(f1));
+      unpack2(mul2(ff, slack), f0, f1);
+      f(4 * h + 2 * k, n0, n0 <= f0);
+      f(4 * h + 2 * k + 1, n1, n1 <= f1);
+    }
+    // keeps the second half's loads after the first half's tests (fewer
+    // live registers)
+    asm volatile("" ::: "memory");
+  }
+}
+
+// A stack entry is a child reference with its entry distance, or, with
+// kGroupBit set, a node some of whose hit children were not visited yet:
+// their mask in the 8 low bits of t, whose other bits are a lower bound of
+// their entry distances.
+constexpr uint32_t kGroupBit = 0x40000000u;  // node indices stay below it (kMaxSlots)
+constexpr uint32_t kNoRef = kEmptyChild;
+
+// What a lane of a persistent kernel does next, as the addend that counts
+// the lanes of each kind in one warp sum (a byte per kind).
+constexpr uint32_t kLanePop = 0u;             // takes the next stack entry
+constexpr uint32_t kLaneNode = 1u;            // tests the children of node `ref`
+constexpr uint32_t kLaneTri = 1u << 8;        // tests the triangles of mesh leaf `ref`
+constexpr uint32_t kLaneObj = 1u << 16;       // tests the object of instance leaf `ref`
+constexpr uint32_t kLaneDone = 1u << 24;      // its ray is finished
+constexpr uint32_t kLaneIdle = (1u << 24) | (1u << 31);  // has no ray (bits 30 and 31 of the sum are not read)
+
+// trace_tlas as a resumable state machine: trace_begin sets up a ray, then
+// trace_pop and one of trace_node, trace_leaf and trace_object advance it.
+// The persistent trace kernels call these in a loop shared by the whole warp
+// and give a lane a new ray once its ray is finished.
+//
+// The state is what has to survive between steps and no more: the closest
+// hit's face, barycentrics and point go to the hit record when the hit is
+// accepted, the ray's moment is computed per leaf, and what a query skips
+// follows from its phase.  The closest-hit kernel so fits 80 registers (6
+// blocks per SM) without spills; with the whole hit in registers it spilled
+// 150 B there and ran best at 96 (benchmark frame: closest-hit 145 ms, with
+// the short state 127 ms).
+struct TraceState {
+  // the ray of the current level: the world ray, or the mesh-local ray while
+  // a mesh is entered, when the world ray waits in shared memory
+  // (SplitStack::ws)
+  Ray w;
+  float z;         // closest hit so far (the bound of an any-hit query)
+  uint32_t obj;    // its object, UINT32_MAX: none
+  float exit;      // where the ray leaves its bounds if they contain the ray origin, else -1
+  float cur_exit;  // the same for the entered mesh
+  uint32_t cur;    // object of the entered mesh
+  uint32_t n_inside;  // meshes met whose bounds contain the ray origin
+  uint32_t kind;   // what the lane does next (kLane*)
+  uint32_t ref;    // the node or leaf it does that with
+  int base;        // stack height at which the entered mesh is done; -1 in world space
+  bool lowered;    // z was lowered for the entered mesh (it loses ties)
+  // 1: closest hit; 2: any hit among the objects below wobj; 3: closest hit
+  // without object wobj (any-hit kernels: 1, any hit without object wobj)
+  int phase;
+  uint32_t wobj;
+};
+
+// The next step: node or leaf `ref`, or the stack's top if it is kNoRef.
+__device__ __forceinline__ void trace_next(TraceState& t, uint32_t ref) {
+  t.ref = ref;
+  t.kind = (ref & kLeafBit) ? (t.base >= 0 ? kLaneTri : kLaneObj) : kLaneNode;
+  if (ref == kNoRef) t.kind = kLanePop;
+}
+
+__device__ __forceinline__ void trace_begin(const DevScene& S, TraceState& t, SplitStack& st) {
+  t.obj = UINT32_MAX;
+  t.exit = -1.f;
+  t.lowered = false;
+  t.base = -1;
+  t.n_inside = 0;
+  st.sp = 0;
+  t.kind = kLaneDone;
+  // without objects there is no instance BVH: every ray misses
+  if (S.n_objects != 0 && segment_box_entry(S.tlas_bounds, t.w, t.z) != kFltMax) trace_next(t, S.tlas_root);
+}
+
+// Takes the next entry from the stack, leaving the entered mesh when its
+// entries are used up.  An entry beyond the closest hit is dropped (the lane
+// pops again).  For a node, `todo` is the mask of the children to test.
 template <bool ANY>
-__device__ __forceinline__ bool trace_step(const DevScene& S, TraceState& t, SplitStack& st,
-                                           TravStats& ts) {
-  if (st.sp == 0) return true;
-  bool const any = ANY || t.any;
-  StackEntry const e = st.pop();
-  HitRec& h = t.h;
-  if (e.ref == kMarker) {
-    t.in_mesh = false;
-    if (t.lowered && h.obj != t.cur) h.z = t.zs;
+__device__ __forceinline__ void trace_pop(const DevScene& S, TraceState& t, SplitStack& st, uint32_t& todo) {
+  if (st.sp <= t.base) {
+    // the mesh is done: back to the world ray, and to the distance before it
+    // was lowered unless the mesh was hit
+    t.base = -1;
+    if (!ANY && t.lowered && t.obj != t.cur) t.z = next_float(t.z);
     t.lowered = false;
     t.w.p = f3{st.ws[0], st.ws[128], st.ws[2 * 128]};
     t.w.u = f3{st.ws[3 * 128], st.ws[4 * 128], st.ws[5 * 128]};
     t.w.inv = f3{st.ws[6 * 128], st.ws[7 * 128], st.ws[8 * 128]};
-    return st.sp == 0;
   }
-  if (e.t > h.z * kTravSlack) return st.sp == 0;
-  if (!(e.ref & kLeafBit)) {
-    ts.nodes++;
-    // children near to far, except in the shadow kernel: its answer does not
-    // depend on the order, and sorting costs it more than it saves.  (The
-    // closest-hit kernel's own any-hit queries are faster sorted.)
-    if (!push_children_split<true>(S.nodes[e.ref], t.w, h.z, st, !ANY)) {
-      ts.flags |= 1u;
-      return true;
+  if (st.sp == 0) {
+    t.kind = kLaneDone;
+    return;
+  }
+  StackEntry const e = st.pop();
+  uint32_t ref = e.ref;
+  if (ANY) {
+    if (!(ref & kLeafBit) && (ref & kGroupBit)) {
+      uint32_t const m = __float_as_uint(e.t);
+      uint32_t const c = 31u - __clz(m);
+      uint32_t const rest = m ^ (1u << c);
+      if (rest) st.push(StackEntry{ref, __uint_as_float(rest)});
+      ref = S.nodes[ref ^ kGroupBit].child[c];
     }
-    return st.sp == 0;
+  } else {
+    if (e.t > t.z * kTravSlack) return;
+    if (!(ref & kLeafBit) && (ref & kGroupBit)) {
+      todo = __float_as_uint(e.t) & 0xFFu;
+      ref ^= kGroupBit;
+    }
   }
-  uint32_t const cnt = ((e.ref >> 28) & 7u) + 1u;
-  uint32_t const slot = e.ref & kSlotMask;
-  if (t.in_mesh) {
-    for (uint32_t k = 0; k < cnt; k++) {
-      const TriSlot& T = S.tris[slot + k];
-      ts.tris++;
-      float tt, b0, b1, b2;
-      Ray const& lr = t.w;
-      if (tri_test(T, lr, t.mr, h.z, tt, b0, b1, b2)) {
-        h.z = tt;
-        h.obj = t.cur;
-        h.face = __float_as_uint(T.v0[3]);
-        h.b0 = b0;
-        h.b1 = b1;
-        h.b2 = b2;
-        h.pl = ray_at(lr, tt);
-        h.inside = t.cur_inside;
-        h.exit = t.cur_exit;
-        t.hit_any = true;
-        if (any) return true;
+  trace_next(t, ref);
+}
+
+// Tests the children of node t.ref that are in `todo`.
+//
+// Closest-hit rays visit a node's hit children from near to far without
+// sorting them: the nearest is the next step's (no stack access), the second
+// is pushed with its distance, and the others wait as a group entry.  Once
+// that is popped and its bound is not beyond the closest hit, the node's
+// remaining children are tested again, against the closest hit by then.  Few
+// nodes have a third hit child that is still wanted (4 % more node tests on
+// the benchmark frame), and the order is that of a full sort by (distance
+// without its 3 low bits, child): finding the two nearest of 8 takes 17
+// min/max operations where a sorting network takes 38 and up to 8 pushes.
+// Shadow rays visit them from the last to the first (their answer does not
+// depend on the order, and distance order is slower), as one group.
+template <bool ANY>
+__device__ __forceinline__ void trace_node(const DevScene& S, TraceState& t, SplitStack& st, uint32_t todo) {
+  uint32_t const ref = t.ref;
+  uint32_t next = kNoRef;
+  const WideNode& nd = S.nodes[ref];
+  if (st.sp + 2 > kSplitCap) {
+    st.flags |= kTravOverflow;
+    t.kind = kLaneDone;
+    return;
+  }
+  uint32_t m = 0;
+  if (ANY) {
+    node_children(nd, t.w, t.z, [&](int c, float, bool hit) {
+      if (hit) m |= 1u << c;
+    });
+    if (m) {
+      uint32_t const c = 31u - __clz(m);
+      uint32_t const rest = m ^ (1u << c);
+      if (rest) st.push(StackEntry{ref | kGroupBit, __uint_as_float(rest)});
+      next = nd.child[c];
+    }
+    trace_next(t, next);
+    return;
+  }
+  uint32_t key[8];
+  node_children(nd, t.w, t.z, [&](int c, float tc, bool hit) {
+    key[c] = hit ? ((__float_as_uint(tc) & ~7u) | uint32_t(7 - c)) : 0xFFFFFFFFu;
+    if (hit) m |= 1u << c;
+  });
+  if (todo != 0xFFu) {
+    m &= todo;
+#pragma unroll
+    for (int c = 0; c < 8; c++)
+      if (!((todo >> c) & 1u)) key[c] = 0xFFFFFFFFu;
+  }
+  // the two smallest keys
+  uint32_t lo[4], hi[4];
+#pragma unroll
+  for (int k = 0; k < 4; k++) {
+    lo[k] = min(key[2 * k], key[2 * k + 1]);
+    hi[k] = max(key[2 * k], key[2 * k + 1]);
+  }
+#pragma unroll
+  for (int n = 2; n > 0; n >>= 1)
+#pragma unroll
+    for (int k = 0; k < n; k++) {
+      uint32_t const a = max(lo[k], lo[k + n]);
+      lo[k] = min(lo[k], lo[k + n]);
+      hi[k] = __vimin3_u32(a, hi[k], hi[k + n]);
+    }
+  if (m) {
+    uint32_t const c1 = 7u - (lo[0] & 7u);
+    next = nd.child[c1];
+    m ^= 1u << c1;
+    if (m) {
+      uint32_t const c2 = 7u - (hi[0] & 7u);
+      uint32_t const ref2 = nd.child[c2];
+      m ^= 1u << c2;
+      if (m) st.push(StackEntry{ref | kGroupBit, __uint_as_float((hi[0] & ~0xFFu) | m)});
+      st.push(StackEntry{ref2, __uint_as_float(hi[0] & ~7u)});
+    }
+  }
+  trace_next(t, next);
+}
+
+// Tests the triangles of mesh leaf t.ref.  accept(face, b0, b1, b2, point,
+// distance) records a closer hit.
+template <bool ANY, class A>
+__device__ __forceinline__ void trace_leaf(const DevScene& S, TraceState& t, uint32_t& tris, A accept) {
+  bool const any = ANY || t.phase == 2;
+  uint32_t const cnt = ((t.ref >> 28) & 7u) + 1u;
+  uint32_t const slot = t.ref & kSlotMask;
+  t.kind = kLanePop;
+  f3 const mr = cross3(t.w.p, t.w.u);
+  for (uint32_t k = 0; k < cnt; k++) {
+    const TriSlot& T = S.tris[slot + k];
+    tris++;
+    float tt, b0, b1, b2;
+    if (tri_test(T, t.w, mr, t.z, tt, b0, b1, b2)) {
+      t.obj = t.cur;
+      if (any) {
+        t.kind = kLaneDone;
+        return;
       }
+      t.z = tt;
+      t.exit = t.cur_exit;
+      accept(__float_as_uint(T.v0[3]), b0, b1, b2, ray_at(t.w, tt), tt);
     }
-    return st.sp == 0;
   }
+}
+
+// Tests the object of instance leaf t.ref (the rest of the leaf waits on the
+// stack): a sphere or plane in full, a mesh by its bounds, after which the
+// next step enters its tree.
+template <bool ANY, class A>
+__device__ __forceinline__ void trace_object(const DevScene& S, TraceState& t, SplitStack& st, uint32_t& insts,
+                                             A accept) {
+  bool const any = ANY || t.phase == 2;
+  uint32_t const cnt = ((t.ref >> 28) & 7u) + 1u;
+  uint32_t const slot = t.ref & kSlotMask;
+  t.kind = kLanePop;
   uint32_t const i = S.tlas_objects[slot];
   if (cnt > 1) {
     if (st.sp + 1 > kSplitCap) {
-      ts.flags |= 1u;
-      return true;
+      st.flags |= kTravOverflow;
+      t.kind = kLaneDone;
+      return;
     }
-    st.push(StackEntry{kLeafBit | ((cnt - 2u) << 28) | (slot + 1u), e.t});
+    st.push(StackEntry{kLeafBit | ((cnt - 2u) << 28) | (slot + 1u), 0.f});
   }
-  if (i == t.skip || i >= t.ilimit) return st.sp == 0;
-  ts.insts++;
+  if (ANY ? i == t.wobj : (t.phase != 1 && (t.phase == 2 ? i >= t.wobj : i == t.wobj))) return;
+  insts++;
   const DevObject& ob = S.objects[i];
-  bool const low = !any && h.obj != UINT32_MAX && i < h.obj;
-  float const z_saved = h.z;
-  if (low) h.z = prev_float(z_saved);
+  bool const low = !any && t.obj != UINT32_MAX && i < t.obj;
+  // a lower-index object loses ties: it has to be hit below the next float
+  float const z = low ? prev_float(t.z) : t.z;
   Ray const li = to_local(ob, t.w);
   if (ob.type != LGPU_OBJ_TRIMESH) {
     float tt;
     f3 x;
     bool hit;
     if (ob.type == LGPU_OBJ_SPHERE) {
-      hit = sphere_test(li, h.z, tt);
+      hit = sphere_test(li, z, tt);
       if (hit) x = ray_at(li, tt);
     } else {
-      hit = plane_test(li, h.z, tt, x);
+      hit = plane_test(li, z, tt, x);
     }
     if (hit) {
-      h.z = tt;
-      h.obj = i;
-      h.face = UINT32_MAX;
-      h.pl = x;
-      h.inside = false;
-      t.hit_any = true;
-      if (any) return true;
-    } else if (low) {
-      h.z = z_saved;
+      t.obj = i;
+      if (any) {
+        t.kind = kLaneDone;
+        return;
+      }
+      t.z = tt;
+      t.exit = -1.f;
+      accept(UINT32_MAX, 0.f, 0.f, 0.f, x, tt);
     }
-    return st.sp == 0;
+    return;
   }
   const DevMesh& m = S.meshes[ob.mesh];
   bool inside;
   float ex;
-  float r0 = aabb_scalar(m.bounds, li, h.z, inside, ex);
-  if (r0 != kFltMax && inside) t.n_inside++;
-  if (r0 != kFltMax && !any && inside) r0 = kBias;
-  if (r0 == kFltMax || r0 > h.z) {
-    if (low) h.z = z_saved;
-    return st.sp == 0;
-  }
-  if (st.sp + 2 > kSplitCap) {
-    ts.flags |= 1u;
-    return true;
-  }
+  float r0 = aabb_scalar(m.bounds, li, z, inside, ex);
+  if (!ANY && r0 != kFltMax && inside) t.n_inside++;
+  if (!any && r0 != kFltMax && inside) r0 = kBias;
+  if (r0 == kFltMax || r0 > z) return;
   st.ws[0] = t.w.p.x;
   st.ws[128] = t.w.p.y;
   st.ws[2 * 128] = t.w.p.z;
@@ -434,16 +633,12 @@ __device__ __forceinline__ bool trace_step(const DevScene& S, TraceState& t, Spl
   st.ws[7 * 128] = t.w.inv.y;
   st.ws[8 * 128] = t.w.inv.z;
   t.w = li;
-  t.mr = cross3(li.p, li.u);
+  t.z = z;
   t.cur = i;
-  t.cur_inside = inside;
-  t.cur_exit = ex;
-  t.zs = z_saved;
+  t.cur_exit = inside ? ex : -1.f;
   t.lowered = low;
-  t.in_mesh = true;
-  st.push(StackEntry{kMarker, 0.f});
-  st.push(StackEntry{m.trav_root, r0});
-  return false;
+  t.base = st.sp;
+  trace_next(t, m.trav_root);
 }
 
 // intersect::scene for the wavefront kernels: the instance BVH through
