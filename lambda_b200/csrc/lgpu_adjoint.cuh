@@ -392,8 +392,8 @@ cudaError_t replay_chunk(const OneJob& jobs, WaveState& w, uint64_t c0, uint32_t
     // one block per queue chunk (see wave_chunk)
     wf_shade_adjoint<K><<<(wi.cap + 127) / 128, 128, 0, st>>>(jobs, wi, g);
     run->end(2, st);
-    // plan, generate, trace (+ fallback), shade
-    run->total += linear ? 4 : 5;
+    // plan, generate, shade
+    run->total += 3 + closest_launches(jobs, linear);
   });
 }
 

@@ -485,9 +485,11 @@ int batch_impl(lgpu_ctx* ctx, const lgpu_job* jobs, uint32_t n, float* const* d_
   std::vector<uint64_t> items(n + 1);
   std::vector<uint32_t> pixels(n + 1);
   uint64_t g = 0, px = 0;
+  uint32_t max_objects = 0;
   for (uint32_t k = 0; k < n; k++) {
     DevJob& d = hj[k];
     d.S = ctx->slots[jobs[k].scene].S;
+    max_objects = std::max(max_objects, d.S.n_objects);
     d.a = render_args(&jobs[k].params, d.S);
     uint32_t th = 0;
     job_rect(jobs[k], d.S.cam, d.col0, d.row0, d.tile_w, th);
@@ -525,8 +527,8 @@ int batch_impl(lgpu_ctx* ctx, const lgpu_job* jobs, uint32_t n, float* const* d_
   e = ctx->keep_counters ? cudaSuccess : cudaMemsetAsync(ctx->counters, 0, 3 * sizeof(DevCounters), st);
   if (e == cudaSuccess) e = cudaEventRecord(ctx->ev0, st);
   if (e == cudaSuccess)
-    e = launch_batch(ctx->S.hero_k, ctx->jobs.ptr, ctx->job_items.ptr, ctx->job_pixels.ptr, n, g, chunk, linear,
-                     &ws, ctx->counters, st, &ctx->launch);
+    e = launch_batch(ctx->S.hero_k, ctx->jobs.ptr, ctx->job_items.ptr, ctx->job_pixels.ptr, n, max_objects, g, chunk,
+                     linear, &ws, ctx->counters, st, &ctx->launch);
   if (e == cudaSuccess) e = cudaEventRecord(ctx->ev1, st);
   // the host tables must outlive their asynchronous copies
   if (e == cudaSuccess) e = cudaStreamSynchronize(st);
@@ -1227,8 +1229,7 @@ int trace_impl(lgpu_ctx* ctx, const float* rays, const float* tmax, const uint32
   if (e == cudaSuccess) e = cudaEventRecord(ctx->ev0, st);
   ctx->launch.reset(false);
   uint64_t const chunks = (n + cap - 1) / cap;
-  // setup, load, store + the traversal (persistent + fallback, or linear)
-  ctx->launch.total = chunks * (any ? 4 : ((flags & LGPU_FLAG_REFERENCE_ORDER) || ctx->S.n_objects <= 4 ? 4 : 5));
+  ctx->launch.total = chunks * trace_launches(ctx->S, any, flags);
   for (uint64_t c0 = 0; c0 < n && e == cudaSuccess; c0 += cap) {
     uint32_t const m = uint32_t(n - c0 < cap ? n - c0 : cap);
     e = cudaMemcpyAsync(ctx->rays.ptr, rays + 6 * c0, 6 * size_t(m) * sizeof(float), cudaMemcpyHostToDevice, st);

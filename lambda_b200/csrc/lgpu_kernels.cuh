@@ -201,6 +201,7 @@ struct OneJob {
   RenderArgs a;
   uint32_t npix;
   float* out;
+  uint32_t max_objects() const { return S.n_objects; }
   __device__ __forceinline__ const DevScene& scene(uint32_t) const { return S; }
   __device__ __forceinline__ const RenderArgs& args(uint32_t) const { return a; }
   __device__ __forceinline__ uint32_t job_of_item(uint64_t) const { return 0; }
@@ -219,6 +220,8 @@ struct JobTable {
   const uint64_t* item_bases;  // n + 1 entries, the last is the total
   const uint32_t* pix_bases;   // n + 1 entries
   uint32_t n;
+  uint32_t objects;            // of the job's scene that has the most
+  uint32_t max_objects() const { return objects; }
   __device__ __forceinline__ const DevScene& scene(uint32_t j) const { return d[j].S; }
   __device__ __forceinline__ const RenderArgs& args(uint32_t j) const { return d[j].a; }
   // the job whose range holds item g / pixel gp (binary search)
@@ -259,21 +262,23 @@ struct JobTable {
 // (any = false) or, for shadow rays with their distance bound and object to
 // skip, whether each is occluded into d_hit_any (any = true).
 size_t trace_wave_layout(uint8_t* base, uint32_t cap, WaveState& ws);
+uint32_t trace_launches(const DevScene& S, bool any, uint32_t flags);  // kernels of one chunk
 cudaError_t launch_trace_chunk(const DevScene& S, WaveState& w, const float* d_rays, const float* d_tmax,
                                const uint32_t* d_skip, uint32_t n, bool any, uint32_t flags,
                                lgpu_hit* d_hits, uint8_t* d_hit_any, const WaveConfig& cfg, DevCounters* d_cnt,
                                cudaStream_t st);
 
 // Batched render of the jobs of `table` (n jobs, n_items work items,
-// n_pix pixels in all) with the wavefront kernels.
+// n_pix pixels in all; max_objects in the largest scene) with the wavefront
+// kernels.
 cudaError_t launch_batch(uint32_t hero_k, const DevJob* d_jobs, const uint64_t* d_item_bases,
-                         const uint32_t* d_pix_bases, uint32_t n_jobs, uint64_t n_items,
+                         const uint32_t* d_pix_bases, uint32_t n_jobs, uint32_t max_objects, uint64_t n_items,
                          uint64_t chunk_items, bool linear, WaveState* wave, DevCounters* d_cnt,
                          cudaStream_t st, WaveLaunch* run);
 template <int K>
 cudaError_t launch_batch_k(const DevJob* d_jobs, const uint64_t* d_item_bases, const uint32_t* d_pix_bases,
-                           uint32_t n_jobs, uint64_t n_items, uint64_t chunk_items, bool linear,
-                           WaveState* wave, DevCounters* d_cnt, cudaStream_t st, WaveLaunch* run);
+                           uint32_t n_jobs, uint32_t max_objects, uint64_t n_items, uint64_t chunk_items,
+                           bool linear, WaveState* wave, DevCounters* d_cnt, cudaStream_t st, WaveLaunch* run);
 
 // Renders with the wavefront kernels when wave != nullptr, else with the
 // one-thread-per-pixel megakernel.  d_cnt points at 3 counter records:

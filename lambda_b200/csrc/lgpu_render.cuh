@@ -163,8 +163,14 @@ void launch_closest(const J& jobs, const WaveState& w, const WaveGrids& g, bool 
     wf_trace<J><<<g.trace, 128, kTraceSmem, st>>>(jobs, w, cnt);
   } else {
     wf_trace_persistent<false, K, J><<<g.ptrace, 128, kTraceSmem, st>>>(jobs, w, cnt);
-    wf_trace_fallback<J><<<g.fb, 128, 0, st>>>(jobs, w, cnt);
+    if (jobs.max_objects() > kMaxLoopObjects) wf_trace_fallback<J><<<g.fb, 128, 0, st>>>(jobs, w, cnt);
   }
+}
+
+// Kernel launches of launch_closest.
+template <class J>
+uint32_t closest_launches(const J& jobs, bool linear) {
+  return !linear && jobs.max_objects() > kMaxLoopObjects ? 2 : 1;
 }
 
 // Swaps the current and next queue, and the shadow contributions of this
@@ -289,8 +295,8 @@ cudaError_t wave_chunk(const J& jobs, WaveState& w, uint64_t c0, uint32_t total,
     if (linear) wf_shadow<K, J><<<g.shadow, 128, kTraceSmem, st>>>(jobs, wi, c_shadow);
     else wf_trace_persistent<true, K, J><<<g.pshadow, 128, kTraceSmem, st>>>(jobs, wi, c_shadow);
     run->end(1, st);
-    // finish, plan, generate, trace (+ fallback), shade (3), shadow
-    run->total += linear ? 8 : 9;
+    // finish, plan, generate, shade (3), shadow
+    run->total += 7 + closest_launches(jobs, linear);
   });
   if (e != cudaSuccess) return e;
   wf_finish<K, J><<<g.fin, 256, 0, st>>>(jobs, w, d_cnt);
@@ -344,9 +350,9 @@ cudaError_t launch_render_k(const DevScene& S, const RenderArgs& a, WaveState* w
 
 template <int K>
 cudaError_t launch_batch_k(const DevJob* d_jobs, const uint64_t* d_item_bases, const uint32_t* d_pix_bases,
-                           uint32_t n_jobs, uint64_t n_items, uint64_t chunk_items, bool linear,
-                           WaveState* wave, DevCounters* d_cnt, cudaStream_t st, WaveLaunch* run) {
-  JobTable const jobs{d_jobs, d_item_bases, d_pix_bases, n_jobs};
+                           uint32_t n_jobs, uint32_t max_objects, uint64_t n_items, uint64_t chunk_items,
+                           bool linear, WaveState* wave, DevCounters* d_cnt, cudaStream_t st, WaveLaunch* run) {
+  JobTable const jobs{d_jobs, d_item_bases, d_pix_bases, n_jobs, max_objects};
   return run_wave<K>(jobs, *wave, n_items, chunk_items, linear, d_cnt, st, run);
 }
 

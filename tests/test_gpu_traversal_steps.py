@@ -26,7 +26,7 @@ def crowded(out_dir, n):
         sc = json.load(f)
     rng = np.random.default_rng(5)
     for o in sc["objects"][1:]:
-        s = float(rng.uniform(0.3, 1.4))
+        s = float(rng.uniform(0.3, 1.4)) * (1.0 if n < 100 else 0.25)
         o["transform"] = {"scale": [s, s * float(rng.uniform(0.3, 1.0)), s],
                           "rotate": {"axis": [float(x) for x in rng.normal(size=3)],
                                      "degrees": float(rng.uniform(0, 360))},
@@ -47,7 +47,9 @@ def rays_of(n, seed):
     return np.concatenate([o, d], axis=1).astype(np.float32)
 
 
-@pytest.fixture(scope="module", params=[5, 40])
+# 5 and 40 objects: one and two groups of the in-kernel object loop; 1100: the
+# separate launch for larger scenes
+@pytest.fixture(scope="module", params=[5, 40, 1100])
 def ctx(request, tmp_path_factory):
     from lambda_b200.renderer import Context
     from lambda_b200.scene import load_nls
@@ -65,6 +67,10 @@ def test_closest_and_any(ctx, n):
     # another face of a shared edge may be reported at an exactly equal
     # distance (about one ray in a million)
     assert np.count_nonzero(a["obj"] != b["obj"]) + np.count_nonzero(a["face"] != b["face"]) <= n // 50000
+    if n == 200003:
+        assert ctx.stats()["device_checks"] == 0
+        ctx.trace(rays)
+        assert ctx.stats()["order_rays"] > 0  # the object loop was taken
     hit = a["obj"] != MISS
     assert n < 100 or 0.05 < hit.mean() < 0.95
     # shadow rays just short of, at and beyond the closest hit, and one that
