@@ -205,16 +205,9 @@ __global__ void __launch_bounds__(256) wf_replay_generate(OneJob jobs, WaveState
                       P.z + dd * (Fx.z * la + Fy.z * lb)};
     f3 const dir = fnorm(f3{wij.x - wkl.x, wij.y - wkl.y, wij.z - wkl.z});
     float const hero = S.lambda_inf + omega * lgpu_flt(&rng);
-    in.ray[0 * cap + p] = wkl.x;
-    in.ray[1 * cap + p] = wkl.y;
-    in.ray[2 * cap + p] = wkl.z;
-    in.ray[3 * cap + p] = dir.x;
-    in.ray[4 * cap + p] = dir.y;
-    in.ray[5 * cap + p] = dir.z;
-    in.rng[p] = rng;
-    in.hero[p] = hero;
-    in.depth[p] = 0;
-    in.item[p] = q;
+    in.ra[p] = make_float4(wkl.x, wkl.y, wkl.z, dir.x);
+    in.rb[p] = make_float4(dir.y, dir.z, hero, __uint_as_float(0u));
+    in.rc[p] = make_uint4(uint32_t(rng), uint32_t(rng >> 32), q, kNoShadow);
     const float* dI = g.dimg + (size_t(H - i - 1) * W + j) * 3;
     float const dR = dI[0], dG = dI[1], dB = dI[2];
     // dLoss/dXYZ through the XYZ -> linear RGB matrix of finalize
@@ -222,12 +215,17 @@ __global__ void __launch_bounds__(256) wf_replay_generate(OneJob jobs, WaveState
     float const dY = -1.5371385f * dR + 1.8760108f * dG - 0.2040259f * dB;
     float const dZ = -0.4985314f * dR + 0.0415560f * dG + 1.0572252f * dB;
 #pragma unroll
-    for (int kk = 0; kk < K; kk++) {
-      float X = 0.f, Y = 0.f, Z = 0.f;
-      splat_xyz(S, hero_lambda(S, hero, step, kk), 1.f, X, Y, Z);
-      in.beta[kk * cap + p] = 1.f;
-      in.acc[kk * cap + p] = w.ltot[size_t(q) * K + kk];
-      in.gw[kk * cap + p] = (dX * X + dY * Y + dZ * Z) * scale;
+    for (int kq = 0; kq < K / 4; kq++) {
+      float gw[4];
+#pragma unroll
+      for (int j = 0; j < 4; j++) {
+        float X = 0.f, Y = 0.f, Z = 0.f;
+        splat_xyz(S, hero_lambda(S, hero, step, 4 * kq + j), 1.f, X, Y, Z);
+        gw[j] = (dX * X + dY * Y + dZ * Z) * scale;
+      }
+      in.beta[kq * cap + p] = make_float4(1.f, 1.f, 1.f, 1.f);
+      in.acc[kq * cap + p] = w.ltot[size_t(q) * (K / 4) + kq];
+      in.gw[kq * cap + p] = make_float4(gw[0], gw[1], gw[2], gw[3]);
     }
   }
 }
@@ -256,18 +254,21 @@ __global__ void __launch_bounds__(128, 10) wf_shade_adjoint(OneJob jobs, WaveSta
     // d ln w_L / dα and d ln w_mat / dα of the MIS weights (below)
     float dlw_L = 0.f, dlw_mat = 0.f;
     uint64_t rng = 0;
-    uint32_t mat = 0, light = 0, depth = 0;
+    uint32_t mat = 0, light = 0, depth = 0, item = 0;
     bool front = true;
     MatSample ms;
     ms.ok = false;
     BsdfScalars bl{};
     if (live) {
-      hero = in.hero[i];
-      depth = in.depth[i];
+      float4 const rb = in.rb[i];
+      uint4 const rc = in.rc[i];
+      hero = rb.z;
+      depth = __float_as_uint(rb.w);
+      item = rc.z;
       uint32_t const obj = w.hobj[i];
       if (obj != UINT32_MAX) {
         HitRec const h = load_hit(w, i, obj);
-        Ray const r = load_ray(in.ray, cap, i);
+        Ray const r = make_ray(in.ra[i], rb);
         HitInfo const H = finalize_hit(S, r, h);
         f3 const un = fnorm(r.u);
         f3 const o = f3{-un.x, -un.y, -un.z};
@@ -278,7 +279,7 @@ __global__ void __launch_bounds__(128, 10) wf_shade_adjoint(OneJob jobs, WaveSta
         // an emitter ends the path; its radiance is not a parameter
         if (m.type != LGPU_MAT_EMITTER && m.type != LGPU_MAT_DIREMITTER && depth <= a.max_scatter) {
           scatter = true;
-          rng = in.rng[i];
+          rng = (uint64_t(rc.y) << 32) | rc.x;
           light = uint32_t(lgpu_u64(&rng) % uint64_t(S.n_lights));
           float const prob_l = 1.f / float(S.n_lights);
           const lgpu_light& L = S.lights[light];
@@ -314,7 +315,7 @@ __global__ void __launch_bounds__(128, 10) wf_shade_adjoint(OneJob jobs, WaveSta
           lis_scale = ls.scale / (ls.prob * prob_l) * w_L;
           m_scale = ms.ok ? w_mat / ms.prob : 0.f;
           bool const needs_test = stmax >= 0.f;
-          visible = !needs_test || ((w.vis[in.item[i]] >> depth) & 1ull);
+          visible = !needs_test || ((w.vis[item] >> depth) & 1ull);
           cont = ms.ok;
           if (cont) {
             np = H.p;
@@ -328,12 +329,19 @@ __global__ void __launch_bounds__(128, 10) wf_shade_adjoint(OneJob jobs, WaveSta
     const DevMaterial& m = S.mats[mat];
     const lgpu_light& L = S.lights[light];
     float g_d = 0.f, g_alpha = 0.f;
+    float4 bt = make_float4(0.f, 0.f, 0.f, 0.f), gws = bt, rems = bt;
+#pragma unroll 1
     for (int k = 0; k < K; k++) {
+      uint32_t const at = uint32_t(k >> 2) * cap;
+      if ((k & 3) == 0) {
+        bt = in.beta[at + i];
+        gws = in.gw[at + i];
+        rems = in.acc[at + i];
+      }
       float const l = hero_lambda(S, hero, step, k);
       float const x = lam_coord(S, l);
-      float const b = in.beta[k * cap + i];
-      float const gw = in.gw[k * cap + i];
-      float rem = in.acc[k * cap + i];
+      float const gw = gws.x;
+      float b = bt.x, rem = rems.x;
       if (visible && lis_scale != 0.f) {
         float const coef = bsdf_k(S, m, bl, x, l, front);
         float const rad = spec_at(S, L.spectrum, x);
@@ -346,24 +354,24 @@ __global__ void __launch_bounds__(128, 10) wf_shade_adjoint(OneJob jobs, WaveSta
         float const f = mat_mult_k(S, m, ms, x, l, front);
         grad_mult(S, m, ms, x, l, f, gw * rem, g, g_d, g_alpha);
         g_alpha += gw * rem * dlw_mat;
-        out.beta[k * cap + o_pos] = b * (f * m_scale);
-        out.acc[k * cap + o_pos] = rem;
-        out.gw[k * cap + o_pos] = gw;
+        b = b * (f * m_scale);
+      }
+      // the words turn by one wavelength (see wf_shade)
+      bt = make_float4(bt.y, bt.z, bt.w, b);
+      gws = make_float4(gws.y, gws.z, gws.w, gw);
+      rems = make_float4(rems.y, rems.z, rems.w, rem);
+      if (cont && (k & 3) == 3) {
+        out.beta[at + o_pos] = bt;
+        out.acc[at + o_pos] = rems;
+        out.gw[at + o_pos] = gws;
       }
     }
     if (g_d != 0.f && isfinite(g_d)) atomicAdd(g.g_mat + 4 * size_t(mat), g_d);
     if (g_alpha != 0.f && isfinite(g_alpha)) atomicAdd(g.g_mat + 4 * size_t(mat) + 1, g_alpha);
     if (cont) {
-      out.ray[0 * cap + o_pos] = np.x;
-      out.ray[1 * cap + o_pos] = np.y;
-      out.ray[2 * cap + o_pos] = np.z;
-      out.ray[3 * cap + o_pos] = nd.x;
-      out.ray[4 * cap + o_pos] = nd.y;
-      out.ray[5 * cap + o_pos] = nd.z;
-      out.rng[o_pos] = rng;
-      out.hero[o_pos] = hero;
-      out.depth[o_pos] = depth + 1;
-      out.item[o_pos] = in.item[i];
+      out.ra[o_pos] = make_float4(np.x, np.y, np.z, nd.x);
+      out.rb[o_pos] = make_float4(nd.y, nd.z, hero, __uint_as_float(depth + 1));
+      out.rc[o_pos] = make_uint4(uint32_t(rng), uint32_t(rng >> 32), item, kNoShadow);
     }
   }
 }

@@ -252,30 +252,25 @@ struct Carver {
 size_t wave_layout(uint8_t* base, uint32_t cap, uint32_t K, uint32_t npix, uint64_t sbuf_items, bool batch,
                    bool adjoint, bool fp64, WaveState& ws) {
   Carver c{base};
-  size_t const n = cap;
+  size_t const n = cap, kq = K / 4;
   for (PathBuf* pb : {&ws.in, &ws.out}) {
-    pb->ray = c.take<float>(6 * n);
-    pb->rng = c.take<uint64_t>(n);
-    pb->hero = c.take<float>(n);
-    pb->depth = c.take<uint32_t>(n);
-    pb->item = c.take<uint32_t>(n);
+    pb->ra = c.take<float4>(n);
+    pb->rb = c.take<float4>(n);
+    pb->rc = c.take<uint4>(n);
     pb->job = batch ? c.take<uint32_t>(n) : nullptr;
-    pb->beta = c.take<float>(size_t(K) * n);
-    pb->acc = c.take<float>(size_t(K) * n);
-    pb->gw = adjoint ? c.take<float>(size_t(K) * n) : nullptr;
-    pb->sidx = c.take<uint32_t>(n);
+    pb->beta = c.take<float4>(kq * n);
+    pb->acc = c.take<float4>(kq * n);
+    pb->gw = adjoint ? c.take<float4>(kq * n) : nullptr;
   }
   ws.hobj = c.take<uint32_t>(n);
   ws.hita = c.take<float4>(n);
   ws.hitb = c.take<float4>(n);
-  ws.e_acc = c.take<float>(size_t(K) * n);
-  ws.e_hero = c.take<float>(n);
-  ws.e_item = c.take<uint32_t>(n);
-  ws.e_job = batch ? c.take<uint32_t>(n) : nullptr;
-  ws.sray = c.take<float>(8 * n);
-  ws.e_sidx = c.take<uint32_t>(n);
-  ws.s_contrib = c.take<float>(size_t(K) * n);
-  ws.s_prev = c.take<float>(size_t(K) * n);
+  ws.e_acc = c.take<float4>(kq * n);
+  ws.e_rec = c.take<uint4>(n);
+  ws.sa = c.take<float4>(n);
+  ws.sb = c.take<float4>(n);
+  ws.s_contrib = c.take<float4>(kq * n);
+  ws.s_prev = c.take<float4>(kq * n);
   ws.s_vis = c.take<uint8_t>(n);
   ws.s_job = batch ? c.take<uint32_t>(n) : nullptr;
   ws.fb_queue = c.take<uint32_t>(n);
@@ -284,7 +279,7 @@ size_t wave_layout(uint8_t* base, uint32_t cap, uint32_t K, uint32_t npix, uint6
   ws.film = c.take<float>(3 * size_t(npix));
   ws.film64 = fp64 ? c.take<double>(3 * size_t(npix)) : nullptr;
   ws.sbuf = c.take<float>(3 * size_t(sbuf_items));
-  ws.ltot = adjoint ? c.take<float>(size_t(K) * sbuf_items) : nullptr;
+  ws.ltot = adjoint ? c.take<float4>(kq * sbuf_items) : nullptr;
   ws.vis = adjoint ? c.take<uint64_t>(sbuf_items) : nullptr;
   ws.s_item = adjoint ? c.take<uint32_t>(n) : nullptr;
   ws.s_depth = adjoint ? c.take<uint32_t>(n) : nullptr;
@@ -831,6 +826,13 @@ int upload_slot(lgpu_ctx* ctx, SceneSlot& sl, const lgpu_scene& scene_in) {
   S.lambda_sup = scene.spec.lambda_sup;
   // coefficientλ::Δ = (sup-inf)/(n-1) (cg.hpp:246)
   S.lambda_delta = (S.lambda_sup - S.lambda_inf) / float(S.n_bins - 1);
+  {
+    float const prob = 1.f / (S.lambda_sup - S.lambda_inf);
+    auto in_range = [](float x) { return x > 0x1p-40f && x < 0x1p40f; };
+    bool const ok = in_range(S.lambda_delta) && in_range(prob);
+    S.lambda_delta_rcp = ok ? 1.f / S.lambda_delta : 0.f;
+    S.prob_lambda_rcp = ok ? 1.f / prob : 0.f;
+  }
   S.cmf = sl.cmf.ptr;
   S.cam = scene.cam;
   std::memcpy(S.tlas_bounds, L.tlas_bounds, sizeof(S.tlas_bounds));

@@ -20,18 +20,20 @@ struct DevCounters {
 };
 
 // Path state of one queue of the wavefront renderer (lgpu_wave.cuh): path
-// i of the queue at index i of every field, field-major.
+// i of the queue at index i of every field.  A field is a 16-byte word, and
+// the K hero wavelengths of a spectral field are K/4 of them (word q of path
+// i, its wavelengths 4q to 4q+3, at q*cap + i): one access moves four values
+// and, where the paths are read out of queue order, uses half of a 32-byte
+// sector instead of an eighth.
 struct PathBuf {
-  float* ray;       // 6*cap (ox, oy, oz, dx, dy, dz)
-  uint64_t* rng;    // cap
-  float* hero;      // cap
-  uint32_t* depth;  // cap
-  uint32_t* item;   // cap: work item, relative to the first item of the chunk
-  uint32_t* job;    // cap: job of the path (batched renders only)
-  float* beta;      // K*cap
-  float* acc;       // K*cap (path replay: the radiance still to come)
-  float* gw;        // K*cap, path replay: dL/d(radiance) per hero wavelength
-  uint32_t* sidx;   // cap: the path's shadow ray of the last iteration, or kNoShadow
+  float4* ra;       // ray: ox, oy, oz, dx
+  float4* rb;       //   dy, dz; hero wavelength, depth
+  uint4* rc;        // random state (2 words), work item relative to the first of the
+                    // chunk, the path's shadow ray of the last iteration or kNoShadow
+  uint32_t* job;    // job of the path (batched renders only)
+  float4* beta;     // K/4 words
+  float4* acc;      // K/4 words (path replay: the radiance still to come)
+  float4* gw;       // K/4 words, path replay: dL/d(radiance) per hero wavelength
 };
 
 // Counters of the wavefront renderer (WaveState::ctl).
@@ -62,14 +64,13 @@ struct WaveState {
   uint32_t* hobj;      // cap: object each path of `in` hit, UINT32_MAX: none
   float4* hita;        // cap: the hit's face, b0, b1, b2 (written for hits only)
   float4* hitb;        // cap: its local point and distance
-  float* e_acc;        // K*cap: radiance of the paths ended this iteration
-  float* e_hero;       // cap
-  uint32_t* e_item;    // cap
-  uint32_t* e_job;     // cap (batched renders only)
-  float* sray;         // 8*cap shadow rays (ox, oy, oz, dx, dy, dz, tmax, skip)
-  uint32_t* e_sidx;    // cap: the ended path's last shadow ray, or kNoShadow
-  float* s_contrib;    // K*cap: contributions of this iteration's shadow rays
-  float* s_prev;       // K*cap: those of the last iteration (swapped with s_contrib)
+  float4* e_acc;       // K/4*cap: radiance of the paths ended this iteration
+  uint4* e_rec;        // cap: their hero wavelength, work item, last shadow ray or
+                       // kNoShadow, job
+  float4* sa;          // cap shadow rays: ox, oy, oz, dx
+  float4* sb;          // cap:   dy, dz; tmax, object to skip
+  float4* s_contrib;   // K/4*cap: contributions of this iteration's shadow rays
+  float4* s_prev;      // K/4*cap: those of the last iteration (swapped with s_contrib)
   uint8_t* s_vis;      // cap: 1 if the shadow ray reached its light
   uint32_t* s_job;     // cap (batched renders only)
   uint32_t* fb_queue;  // cap: `in` indices re-traced in the reference's object order
@@ -83,7 +84,7 @@ struct WaveState {
   // path replay (lgpu_adjoint): the primal pass records every path's
   // radiance and which of its shadow rays were unoccluded; the replay
   // pass reads them back
-  float* ltot;         // K per work item of the chunk, or nullptr
+  float4* ltot;        // K/4 per work item of the chunk, or nullptr
   uint64_t* vis;       // per work item: bit v set = the shadow ray of vertex v reached its light
   uint32_t* s_item;    // cap: work item of each shadow ray
   uint32_t* s_depth;   // cap: its vertex

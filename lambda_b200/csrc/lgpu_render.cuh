@@ -61,7 +61,7 @@ __global__ void __launch_bounds__(128) render_kernel(DevScene S, RenderArgs a, f
       bool finite = true;
 #pragma unroll
       for (int k = 0; k < K; k++) {
-        float const val = acc[k] / prob_l;
+        float const val = div_by_guarded(acc[k], prob_l, S.prob_lambda_rcp);
         finite = finite && isfinite(val);
         splat_xyz(S, hero_lambda(S, hero, step, k), val, sx, sy, sz);
       }
@@ -182,7 +182,7 @@ inline void swap_queues(WaveState& w) {
   uint32_t* const pc = w.n_in;
   w.n_in = w.n_out;
   w.n_out = pc;
-  float* const sc = w.s_contrib;
+  float4* const sc = w.s_contrib;
   w.s_contrib = w.s_prev;
   w.s_prev = sc;
 }

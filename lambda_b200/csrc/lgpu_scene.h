@@ -110,6 +110,10 @@ struct DevScene {
   uint32_t tlas_max_stack;
   uint32_t n_bins, hero_k;
   float lambda_inf, lambda_sup, lambda_delta;
+  // the correctly rounded reciprocals of lambda_delta and of the hero
+  // wavelength's density 1 / (lambda_sup - lambda_inf), or 0 where div_by
+  // (lgpu_path.cuh) may not use them
+  float lambda_delta_rcp, prob_lambda_rcp;
   const float* cmf;  // 3 * n_bins: X, Y, Z
   lgpu_camera cam;
   float tlas_bounds[6];

@@ -25,21 +25,17 @@ __global__ void trace_setup(WaveState w, uint32_t n, bool any) {
   }
 }
 
-// Rays (6 floats each, AoS) -> the queue's field-major layout; shadow rays
+// Rays (6 floats each) -> the queue's ray words; shadow rays
 // also get their distance bound and object to skip.
 __global__ void __launch_bounds__(256) trace_load(WaveState w, const float* __restrict__ rays,
                                                   const float* __restrict__ tmax,
                                                   const uint32_t* __restrict__ skip, uint32_t n, bool any) {
   uint32_t const i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
-  float* const dst = any ? w.sray : w.in.ray;
-  uint32_t const cap = w.cap;
-#pragma unroll
-  for (int c = 0; c < 6; c++) dst[c * cap + i] = rays[6 * size_t(i) + c];
-  if (any) {
-    dst[6 * cap + i] = tmax[i];
-    dst[7 * cap + i] = __uint_as_float(skip[i]);
-  }
+  const float* const r = rays + 6 * size_t(i);
+  (any ? w.sa : w.in.ra)[i] = make_float4(r[0], r[1], r[2], r[3]);
+  if (any) w.sb[i] = make_float4(r[4], r[5], tmax[i], __uint_as_float(skip[i]));
+  else w.in.rb[i] = make_float4(r[4], r[5], 0.f, 0.f);
 }
 
 // Hit records of the queue -> lgpu_hit (hitinfo, cg.hpp:1138-1149).
@@ -47,11 +43,10 @@ __global__ void __launch_bounds__(128) trace_store(DevScene S, WaveState w, uint
                                                    lgpu_hit* __restrict__ out) {
   uint32_t const i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
-  uint32_t const cap = w.cap;
   uint32_t const obj = w.hobj[i];
   lgpu_hit o;
   if (obj != UINT32_MAX) {
-    HitInfo const H = finalize_hit(S, load_ray(w.in.ray, cap, i), load_hit(w, i, obj));
+    HitInfo const H = finalize_hit(S, load_ray(w.in.ra, w.in.rb, i), load_hit(w, i, obj));
     o.t = H.z;
     o.obj = H.obj;
     o.face = H.face;
@@ -120,12 +115,14 @@ size_t trace_wave_layout(uint8_t* base, uint32_t cap, WaveState& ws) {
   };
   ws = WaveState{};
   ws.cap = cap;
-  ws.in.ray = reinterpret_cast<float*>(take(6 * sizeof(float) * size_t(cap)));
+  ws.in.ra = reinterpret_cast<float4*>(take(sizeof(float4) * size_t(cap)));
+  ws.in.rb = reinterpret_cast<float4*>(take(sizeof(float4) * size_t(cap)));
   ws.hobj = reinterpret_cast<uint32_t*>(take(sizeof(uint32_t) * size_t(cap)));
   ws.hita = reinterpret_cast<float4*>(take(sizeof(float4) * size_t(cap)));
   ws.hitb = reinterpret_cast<float4*>(take(sizeof(float4) * size_t(cap)));
   ws.fb_queue = reinterpret_cast<uint32_t*>(take(sizeof(uint32_t) * size_t(cap)));
-  ws.sray = reinterpret_cast<float*>(take(8 * sizeof(float) * size_t(cap)));
+  ws.sa = reinterpret_cast<float4*>(take(sizeof(float4) * size_t(cap)));
+  ws.sb = reinterpret_cast<float4*>(take(sizeof(float4) * size_t(cap)));
   ws.s_vis = take(size_t(cap));
   ws.ctl = reinterpret_cast<uint32_t*>(take(kCtlWords * sizeof(uint32_t)));
   ws.n_in = ws.ctl + kCtlCountA;

@@ -46,11 +46,14 @@ __device__ __forceinline__ uint32_t warp_append(uint32_t* counter, bool pred) {
   return base + __popc(b & ((1u << lane) - 1u));
 }
 
-__device__ __forceinline__ Ray load_ray(const float* ray, uint32_t cap, uint32_t i) {
-  return make_ray(f3{ray[i], ray[cap + i], ray[2 * cap + i]},
-                  f3{ray[3 * cap + i], ray[4 * cap + i], ray[5 * cap + i]});
+// The ray of path or shadow ray i from its two words (its second word's
+// other half: hero wavelength and depth, or distance bound and object to skip).
+__device__ __forceinline__ Ray make_ray(float4 a, float4 b) {
+  return make_ray(f3{a.x, a.y, a.z}, f3{a.w, b.x, b.y});
 }
-
+__device__ __forceinline__ Ray load_ray(const float4* ra, const float4* rb, uint32_t i) {
+  return make_ray(ra[i], rb[i]);
+}
 // Hit records: the object (UINT32_MAX on a miss) and, for a hit, two
 // 16-byte words, so that a closer hit is recorded by two stores and read
 // back by two loads wherever the path lies in the queue.
@@ -169,17 +172,9 @@ __global__ void __launch_bounds__(256) wf_generate_stream(J jobs, WaveState w, D
                       P.z + dd * (Fx.z * la + Fy.z * lb)};
     f3 const dir = fnorm(f3{wij.x - wkl.x, wij.y - wkl.y, wij.z - wkl.z});
     float const hero = S.lambda_inf + omega * lgpu_flt(&rng);
-    in.ray[0 * cap + p] = wkl.x;
-    in.ray[1 * cap + p] = wkl.y;
-    in.ray[2 * cap + p] = wkl.z;
-    in.ray[3 * cap + p] = dir.x;
-    in.ray[4 * cap + p] = dir.y;
-    in.ray[5 * cap + p] = dir.z;
-    in.rng[p] = rng;
-    in.hero[p] = hero;
-    in.depth[p] = 0;
-    in.item[p] = q;
-    in.sidx[p] = kNoShadow;
+    in.ra[p] = make_float4(wkl.x, wkl.y, wkl.z, dir.x);
+    in.rb[p] = make_float4(dir.y, dir.z, hero, __uint_as_float(0u));
+    in.rc[p] = make_uint4(uint32_t(rng), uint32_t(rng >> 32), q, kNoShadow);
     if (J::kMulti) in.job[p] = jb;
     if (w.vis) w.vis[q] = 0;
     // no spectral state: a path at depth 0 has throughput 1 and no
@@ -191,34 +186,44 @@ __global__ void __launch_bounds__(256) wf_generate_stream(J jobs, WaveState w, D
 }
 
 // Ended paths: radiance splatted to XYZ (addHeroλ(λ, Li/prob),
-// src/renderer.cpp:44) into the path's (sample, pixel) film entry.
+// src/renderer.cpp:44) into the path's (sample, pixel) film entry.  Bound by
+// issue (62 %): four wavelengths per word and loop body (40 registers; all
+// 16 unrolled took 64 and 23 % more time), divisions by the two constants as
+// div_by.  Benchmark frame: 16.0 -> 11.2 ms.
 template <int K, class J>
 __global__ void __launch_bounds__(256) wf_finish(J jobs, WaveState w, DevCounters* cnt) {
   uint32_t const n = w.ctl[kCtlEnded];
   uint32_t const cap = w.cap;
   uint32_t nonfinite = 0;
   for (uint32_t e = blockIdx.x * blockDim.x + threadIdx.x; e < n; e += gridDim.x * blockDim.x) {
-    const DevScene& S = jobs.scene(J::kMulti ? w.e_job[e] : 0u);
+    uint4 const rec = w.e_rec[e];
+    const DevScene& S = jobs.scene(J::kMulti ? rec.w : 0u);
     float const omega = S.lambda_sup - S.lambda_inf;
     float const step = omega / float(K);
     float const prob_l = 1.f / omega;
-    float const hero = w.e_hero[e];
+    float const hero = __uint_as_float(rec.x);
     // the light sample of the path's last vertex, if its shadow ray got through
-    uint32_t const sx_i = w.e_sidx[e];
+    uint32_t const sx_i = rec.z;
     bool const lit = sx_i != kNoShadow && w.s_vis[sx_i];
     float sx = 0.f, sy = 0.f, sz = 0.f;
     bool finite = true;
+#pragma unroll 1
+    for (int q = 0; q < K / 4; q++) {
+      float4 const a4 = w.e_acc[q * cap + e];
+      float4 const p4 = lit ? w.s_prev[q * cap + sx_i] : make_float4(0.f, 0.f, 0.f, 0.f);
+      float acc[4] = {a4.x, a4.y, a4.z, a4.w};
+      float const pend[4] = {p4.x, p4.y, p4.z, p4.w};
 #pragma unroll
-    for (int k = 0; k < K; k++) {
-      float acc = w.e_acc[k * cap + e];
-      if (lit) acc += w.s_prev[k * cap + sx_i];
-      if (w.ltot) w.ltot[size_t(w.e_item[e]) * K + k] = acc;
-      float const val = acc / prob_l;
-      finite = finite && isfinite(val);
-      splat_xyz(S, hero_lambda(S, hero, step, k), val, sx, sy, sz);
+      for (int j = 0; j < 4; j++) {
+        if (lit) acc[j] += pend[j];
+        float const val = div_by_guarded(acc[j], prob_l, S.prob_lambda_rcp);
+        finite = finite && isfinite(val);
+        splat_xyz(S, hero_lambda(S, hero, step, 4 * q + j), val, sx, sy, sz);
+      }
+      if (w.ltot) w.ltot[size_t(rec.y) * (K / 4) + q] = make_float4(acc[0], acc[1], acc[2], acc[3]);
     }
     nonfinite += finite ? 0u : 1u;
-    size_t const o = 3 * size_t(w.e_item[e]);
+    size_t const o = 3 * size_t(rec.y);
     w.sbuf[o] = sx;
     w.sbuf[o + 1] = sy;
     w.sbuf[o + 2] = sz;
@@ -320,7 +325,7 @@ __global__ void __launch_bounds__(128) wf_trace(J jobs, WaveState w, DevCounters
     uint32_t const jb = J::kMulti ? w.in.job[i] : 0u;
     const DevScene& S = jobs.scene(jb);
     bool const ref_order = (jobs.args(jb).flags & LGPU_FLAG_REFERENCE_ORDER) != 0;
-    Ray const r = load_ray(w.in.ray, w.cap, i);
+    Ray const r = load_ray(w.in.ra, w.in.rb, i);
     HitRec h;
     clear_hit(h, kFltMax);
     scene_trace<false>(S, r, h, UINT32_MAX, ref_order, st, lstack, ltstack, ts);
@@ -411,7 +416,7 @@ __global__ void __launch_bounds__(128, ANY ? 7 : 6) wf_trace_persistent(J jobs, 
           bool const ask = t.phase == 1 && t.exit > t.z && t.obj != 0u, again = t.phase == 2 && t.obj != UINT32_MAX;
           if (t.phase != 2) w.hobj[idx] = t.obj;
           if (ask || again) {
-            t.w = load_ray(w.in.ray, cap, idx);
+            t.w = load_ray(w.in.ra, w.in.rb, idx);
             uint32_t const others = t.n_inside;
             if (ask) {
               t.z = prev_float(t.exit);
@@ -469,11 +474,12 @@ __global__ void __launch_bounds__(128, ANY ? 7 : 6) wf_trace_persistent(J jobs, 
           idx = base + k;
           if (J::kMulti) jb = ANY ? w.s_job[idx] : w.in.job[idx];
           if (ANY) {
-            t.w = load_ray(w.sray, cap, idx);
-            t.z = w.sray[6 * cap + idx];
-            t.wobj = __float_as_uint(w.sray[7 * cap + idx]);
+            float4 const b = w.sb[idx];
+            t.w = make_ray(w.sa[idx], b);
+            t.z = b.z;
+            t.wobj = __float_as_uint(b.w);
           } else {
-            t.w = load_ray(w.in.ray, cap, idx);
+            t.w = load_ray(w.in.ra, w.in.rb, idx);
             t.z = kFltMax;
           }
           t.phase = 1;
@@ -520,7 +526,7 @@ __global__ void __launch_bounds__(128) wf_trace_fallback(J jobs, WaveState w, De
   for (uint32_t i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; i < n; i += nwarps) {
     uint32_t const p = w.fb_queue[i];
     const DevScene& S = jobs.scene(J::kMulti ? w.in.job[p] : 0u);
-    Ray const r = load_ray(w.in.ray, w.cap, p);
+    Ray const r = load_ray(w.in.ra, w.in.rb, p);
     HitRec h;
     clear_hit(h, kFltMax);
     h.inside = false;
@@ -633,13 +639,19 @@ __device__ __forceinline__ bool shade_group(uint32_t group) {
   return group != 1u + LGPU_MAT_BLINN && group != 1u + LGPU_MAT_THINFILM;
 }
 
-// Six blocks of 256 per SM (40 registers, with spills) for the first
-// launch: the kernel waits on memory, and more warps hide it better than
-// registers save spill traffic (4 blocks at 64 registers: +18 % shading
-// time, 5: +2 %, 8: +5 %).  The list launches, whose warps are all busy,
-// run 5 (48 registers; 6 and 4: +0.6 % and +0 % shading time).
+// Bound by memory latency (35 % of the issue slots, 2.4 TB/s of path state)
+// and by what the geometry part spills.  So each launch's code knows which
+// materials it can meet, the path's records are written before the
+// wavelength loop (which then keeps only its scalars), and that loop moves
+// 16-byte words of four wavelengths but computes one at a time: unrolled by
+// four, its code overflowed the instruction cache (8 of 23 stalls) and was
+// 17 % slower than 4-byte accesses.  4 blocks of 256 per SM (64 registers)
+// for the first launch and the lists: 5 are 2 % faster on the benchmark
+// frame's first launch but 7 % slower on the box room's; 6 and 5 before.
+// Benchmark frame: first launch 48.2 -> 39.2 ms, Blinn list 16.5 -> 14.9,
+// thin-film list 16.3 -> 14.3; box room 605 -> 472 us.
 template <int K, class J, int MT = -1>
-__global__ void __launch_bounds__(kMaxShadeBlock, (MT == LGPU_MAT_BLINN || MT == LGPU_MAT_THINFILM) ? 5 : 6) wf_shade(J jobs, WaveState w, DevCounters* cnt) {
+__global__ void __launch_bounds__(kMaxShadeBlock, 4) wf_shade(J jobs, WaveState w, DevCounters* cnt) {
   uint32_t const n = *w.n_in;
   uint32_t const cap = w.cap;
   PathBuf const& in = w.in;
@@ -673,7 +685,10 @@ __global__ void __launch_bounds__(kMaxShadeBlock, (MT == LGPU_MAT_BLINN || MT ==
     // type at compile time
     auto material = [&](uint32_t idx) {
       DevMaterial x = S.mats[idx];
-      if (MT == LGPU_MAT_BLINN || MT == LGPU_MAT_THINFILM) x.type = MT;
+      if (kList) x.type = MT;
+      // neither Blinn nor thin film (the compiler then drops their code)
+      if (MT == LGPU_MAT_LAMBERTIAN && (x.type == LGPU_MAT_BLINN || x.type == LGPU_MAT_THINFILM))
+        x.type = LGPU_MAT_MICROFACET;
       return x;
     };
     int kind = kEnd;
@@ -689,12 +704,18 @@ __global__ void __launch_bounds__(kMaxShadeBlock, (MT == LGPU_MAT_BLINN || MT ==
     MatSample ms;
     ms.ok = false;
     BsdfScalars bl{};
+    uint32_t depth = 0, item = 0, prev_s = kNoShadow;
     if (live) {
-      hero = in.hero[i];
+      float4 const rb = in.rb[i];
+      uint4 const rc = in.rc[i];
+      hero = rb.z;
+      depth = __float_as_uint(rb.w);
+      item = rc.z;
+      prev_s = rc.w;
       uint32_t const obj = w.hobj[i];
       if (obj != UINT32_MAX) {
         HitRec const h = load_hit(w, i, obj);
-        Ray const r = load_ray(in.ray, cap, i);
+        Ray const r = make_ray(in.ra[i], rb);
         HitInfo const H = finalize_hit(S, r, h);
         f3 const un = fnorm(r.u);
         f3 const o = f3{-un.x, -un.y, -un.z};
@@ -708,9 +729,9 @@ __global__ void __launch_bounds__(kMaxShadeBlock, (MT == LGPU_MAT_BLINN || MT ==
             float const c = fdot(o, H.F.z);
             g_emit = powf(c >= 0.f ? c : 0.f, m.specular);
           }
-        } else if (in.depth[i] <= a.max_scatter) {
+        } else if (depth <= a.max_scatter) {
           kind = kScatter;
-          rng = in.rng[i];
+          rng = (uint64_t(rc.y) << 32) | rc.x;
           light = uint32_t(lgpu_u64(&rng) % uint64_t(S.n_lights));
           float const prob_l = 1.f / float(S.n_lights);
           const lgpu_light& L = S.lights[light];
@@ -741,83 +762,101 @@ __global__ void __launch_bounds__(kMaxShadeBlock, (MT == LGPU_MAT_BLINN || MT ==
         }
       }
     }
+    // what this launch's materials leave of the BSDF cases and lobes
+    if (MT == LGPU_MAT_LAMBERTIAN) {
+      bl.kind = bl.kind ? 1 : 0;
+      ms.lobe = ms.lobe ? 1 : 0;
+    } else if (MT == LGPU_MAT_BLINN) {
+      bl.kind = bl.kind == 2 ? 2 : 3;
+    } else if (MT == LGPU_MAT_THINFILM) {
+      bl.kind = bl.kind ? 4 : 0;
+      ms.lobe = ms.lobe ? 4 : 0;
+    }
     // compacted appends: next queue, ended list, shadow queue
     bool const ended = live && !cont;
     uint32_t const o_pos = warp_append(w.n_out, cont);
     uint32_t const e_pos = warp_append(w.ctl + kCtlEnded, ended);
     uint32_t const s_pos = warp_append(w.ctl + kCtlShadow, shadow);
     if (!live) continue;
-    float* const acc_dst = cont ? out.acc + o_pos : w.e_acc + e_pos;
-    DevMaterial const m = material(mat);
-    // the light sample of the path's previous vertex, if its shadow ray got
-    // through (recorded by the shadow kernel of the last iteration)
-    uint32_t const prev_s = in.sidx[i];
-    const float* const pend = (prev_s != kNoShadow && w.s_vis[prev_s]) ? w.s_prev + prev_s : nullptr;
-    // a path at depth 0 starts with throughput 1 and no radiance (the
-    // generate kernel writes neither)
-    bool const fresh = in.depth[i] == 0;
-    auto beta_k = [&](int k) { return fresh ? 1.f : in.beta[k * cap + i]; };
-    auto acc_k = [&](int k) { return fresh ? 0.f : in.acc[k * cap + i]; };
-    if (kind == kScatter) {
-      const lgpu_light& L = S.lights[light];
-      for (int k = 0; k < K; k++) {
-        float const l = hero_lambda(S, hero, step, k);
-        float const x = lam_coord(S, l);
-        float const coef = bsdf_k(S, m, bl, x, l, front);
-        float const rad = spec_at(S, L.spectrum, x);
-        float const b = beta_k(k);
-        float const contrib = b * (rad * coef * lis_scale);
-        float acc = acc_k(k);
-        if (pend) acc += pend[k * cap];
-        if (!needs_test) acc += contrib;
-        else if (shadow) w.s_contrib[k * cap + s_pos] = contrib;
-        if (cont) out.beta[k * cap + o_pos] = b * (mat_mult_k(S, m, ms, x, l, front) * m_scale);
-        acc_dst[k * cap] = acc;
-      }
-    } else if (kind == kEmit) {
-      for (int k = 0; k < K; k++) {
-        float const x = lam_coord(S, hero_lambda(S, hero, step, k));
-        float acc = acc_k(k);
-        if (pend) acc += pend[k * cap];
-        acc_dst[k * cap] = acc + beta_k(k) * (spec_at(S, m.spectrum[0], x) * g_emit);
-      }
-    } else {
-#pragma unroll
-      for (int k = 0; k < K; k++) acc_dst[k * cap] = acc_k(k) + (pend ? pend[k * cap] : 0.f);
-    }
+    // the path's records first: the wavelength loop below then has only the
+    // scalars of its spectra to keep in registers
+    uint32_t const s_ref = shadow ? s_pos : kNoShadow;
     if (cont) {
-      out.ray[0 * cap + o_pos] = np.x;
-      out.ray[1 * cap + o_pos] = np.y;
-      out.ray[2 * cap + o_pos] = np.z;
-      out.ray[3 * cap + o_pos] = nd.x;
-      out.ray[4 * cap + o_pos] = nd.y;
-      out.ray[5 * cap + o_pos] = nd.z;
-      out.rng[o_pos] = rng;
-      out.hero[o_pos] = hero;
-      out.depth[o_pos] = in.depth[i] + 1;
-      out.item[o_pos] = in.item[i];
-      out.sidx[o_pos] = shadow ? s_pos : kNoShadow;
+      out.ra[o_pos] = make_float4(np.x, np.y, np.z, nd.x);
+      out.rb[o_pos] = make_float4(nd.y, nd.z, hero, __uint_as_float(depth + 1));
+      out.rc[o_pos] = make_uint4(uint32_t(rng), uint32_t(rng >> 32), item, s_ref);
       if (J::kMulti) out.job[o_pos] = jb;
     } else {
-      w.e_hero[e_pos] = hero;
-      w.e_item[e_pos] = in.item[i];
-      w.e_sidx[e_pos] = shadow ? s_pos : kNoShadow;
-      if (J::kMulti) w.e_job[e_pos] = jb;
+      w.e_rec[e_pos] = make_uint4(__float_as_uint(hero), item, s_ref, jb);
     }
     if (shadow) {
       if (J::kMulti) w.s_job[s_pos] = jb;
       if (w.vis) {
-        w.s_item[s_pos] = in.item[i];
-        w.s_depth[s_pos] = in.depth[i];
+        w.s_item[s_pos] = item;
+        w.s_depth[s_pos] = depth;
       }
-      w.sray[0 * cap + s_pos] = sp.x;
-      w.sray[1 * cap + s_pos] = sp.y;
-      w.sray[2 * cap + s_pos] = sp.z;
-      w.sray[3 * cap + s_pos] = sd.x;
-      w.sray[4 * cap + s_pos] = sd.y;
-      w.sray[5 * cap + s_pos] = sd.z;
-      w.sray[6 * cap + s_pos] = stmax;
-      w.sray[7 * cap + s_pos] = __uint_as_float(sskip);
+      w.sa[s_pos] = make_float4(sp.x, sp.y, sp.z, sd.x);
+      w.sb[s_pos] = make_float4(sd.y, sd.z, stmax, __uint_as_float(sskip));
+    }
+    float4* const acc_dst = cont ? out.acc + o_pos : w.e_acc + e_pos;
+    DevMaterial const m = material(mat);
+    // the light sample of the path's previous vertex, if its shadow ray got
+    // through (recorded by the shadow kernel of the last iteration)
+    const float4* const pend = (prev_s != kNoShadow && w.s_vis[prev_s]) ? w.s_prev + prev_s : nullptr;
+    // a path at depth 0 starts with throughput 1 and no radiance (the
+    // generate kernel writes neither)
+    bool const fresh = depth == 0;
+    auto load_beta = [&](int q) { return fresh ? make_float4(1.f, 1.f, 1.f, 1.f) : in.beta[q * cap + i]; };
+    // the radiance so far, with that light sample
+    auto load_acc = [&](int q) {
+      float4 const v = fresh ? make_float4(0.f, 0.f, 0.f, 0.f) : in.acc[q * cap + i];
+      float4 const p = pend ? pend[q * cap] : make_float4(0.f, 0.f, 0.f, 0.f);
+      return make_float4(v.x + p.x, v.y + p.y, v.z + p.z, v.w + p.w);
+    };
+    if (kind == kScatter) {
+      const lgpu_light& L = S.lights[light];
+      float4 bt = make_float4(0.f, 0.f, 0.f, 0.f), acc = bt, con = bt;
+#pragma unroll 1
+      for (int k = 0; k < K; k++) {
+        if ((k & 3) == 0) {
+          bt = load_beta(k >> 2);
+          acc = load_acc(k >> 2);
+        }
+        float const l = hero_lambda(S, hero, step, k);
+        float const x = lam_coord(S, l);
+        float const coef = bsdf_k(S, m, bl, x, l, front);
+        float const rad = spec_at(S, L.spectrum, x);
+        float const contrib = bt.x * (rad * coef * lis_scale);
+        float const a_k = needs_test ? acc.x : acc.x + contrib;
+        float const b_k = cont ? bt.x * (mat_mult_k(S, m, ms, x, l, front) * m_scale) : 0.f;
+        // the words turn by one wavelength, so one loop body serves all four
+        acc = make_float4(acc.y, acc.z, acc.w, a_k);
+        bt = make_float4(bt.y, bt.z, bt.w, b_k);
+        con = make_float4(con.y, con.z, con.w, contrib);
+        if ((k & 3) == 3) {
+          uint32_t const at = uint32_t(k >> 2) * cap;
+          if (shadow) w.s_contrib[at + s_pos] = con;
+          if (cont) out.beta[at + o_pos] = bt;
+          acc_dst[at] = acc;
+        }
+      }
+    } else if (kind == kEmit) {
+      float4 bt = make_float4(0.f, 0.f, 0.f, 0.f), acc = bt;
+#pragma unroll 1
+      for (int k = 0; k < K; k++) {
+        if ((k & 3) == 0) {
+          bt = load_beta(k >> 2);
+          acc = load_acc(k >> 2);
+        }
+        float const x = lam_coord(S, hero_lambda(S, hero, step, k));
+        float const a_k = acc.x + bt.x * (spec_at(S, m.spectrum[0], x) * g_emit);
+        acc = make_float4(acc.y, acc.z, acc.w, a_k);
+        bt = make_float4(bt.y, bt.z, bt.w, 0.f);
+        if ((k & 3) == 3) acc_dst[uint32_t(k >> 2) * cap] = acc;
+      }
+    } else {
+#pragma unroll
+      for (int q = 0; q < K / 4; q++) acc_dst[q * cap] = load_acc(q);
     }
   }
   (void)cnt;
@@ -841,10 +880,11 @@ __global__ void __launch_bounds__(128) wf_shadow(J jobs, WaveState w, DevCounter
     uint32_t const jb = J::kMulti ? w.s_job[i] : 0u;
     const DevScene& S = jobs.scene(jb);
     bool const ref_order = (jobs.args(jb).flags & LGPU_FLAG_REFERENCE_ORDER) != 0;
-    Ray const r = load_ray(w.sray, cap, i);
+    float4 const b = w.sb[i];
+    Ray const r = make_ray(w.sa[i], b);
     HitRec h;
-    clear_hit(h, w.sray[6 * cap + i]);
-    uint32_t const skip = __float_as_uint(w.sray[7 * cap + i]);
+    clear_hit(h, b.z);
+    uint32_t const skip = __float_as_uint(b.w);
     bool const occ = scene_trace<true>(S, r, h, skip, ref_order, st, lstack, ltstack, ts);
     rays++;
     shadow_done(w, i, !occ);
