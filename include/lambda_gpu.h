@@ -503,10 +503,10 @@ int lgpu_get_stats(const lgpu_ctx* ctx, lgpu_stats* out);
    floats and/or d_out_rgb24 w*h*3 bytes out (either may be NULL), and a
    stream (NULL: the legacy default stream); the call returns when the
    results are written.
-   Scratch: the reduction's per-block partial sums and the exposure live in
-   one file-scope __device__ array of LGPU_NOALLOC_SCRATCH_BYTES bytes that
-   every GPU loading the library holds until exit.  Calls share it: two calls
-   that overlap on the same GPU race and must be serialised by the caller.
+   Scratch: the reduction's per-block partial sums live in one file-scope
+   __device__ array of LGPU_NOALLOC_SCRATCH_BYTES bytes that every GPU
+   loading the library holds until exit.  Calls share it: two calls that
+   overlap on the same GPU race and must be serialised by the caller.
    Every slot a call reads is written by that call first, so nothing needs
    clearing between calls.  The first call on each device looks up the
    array's device address (cudaGetSymbolAddress) with that device current;

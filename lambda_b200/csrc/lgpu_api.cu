@@ -111,7 +111,6 @@ struct lgpu_ctx {
   DevArray<float> tm_in, tm_out;
   DevArray<uint8_t> tm_24;
   DevCounters* counters = nullptr;  // 3 records: all kernels, closest-hit, shadow
-  float* exposure = nullptr;
   WaveLaunch launch;
   bool events_ready = false;
   WaveConfig cfg;     // launch shape of the wavefront
@@ -863,7 +862,6 @@ int lgpu_create(int device, lgpu_ctx** out) {
   if (e == cudaSuccess) e = cudaEventCreateWithFlags(&ctx->ev_fork, cudaEventDisableTiming);
   if (e == cudaSuccess) e = cudaEventCreateWithFlags(&ctx->ev_join, cudaEventDisableTiming);
   if (e == cudaSuccess) e = cudaMalloc(&ctx->counters, 3 * sizeof(DevCounters));
-  if (e == cudaSuccess) e = cudaMalloc(&ctx->exposure, sizeof(float));
   if (e == cudaSuccess) e = cudaMallocHost(&ctx->h_ctl, kCtlWords * sizeof(uint32_t));
   if (e != cudaSuccess) {
     lgpu_destroy(ctx);
@@ -901,7 +899,6 @@ void lgpu_destroy(lgpu_ctx* ctx) {
   ctx->tm_out.release();
   ctx->tm_24.release();
   if (ctx->counters) cudaFree(ctx->counters);
-  if (ctx->exposure) cudaFree(ctx->exposure);
   if (ctx->ev0) cudaEventDestroy(ctx->ev0);
   if (ctx->ev1) cudaEventDestroy(ctx->ev1);
   if (ctx->ev_fork) cudaEventDestroy(ctx->ev_fork);
@@ -1325,7 +1322,7 @@ int lgpu_tonemap(lgpu_ctx* ctx, const float* linrgb, uint64_t w, uint64_t h, flo
   if (e != cudaSuccess) return cuda_fail(ctx, e, "tone-map buffers");
   e = cudaMemcpyAsync(ctx->tm_in.ptr, linrgb, 3 * n * sizeof(float), cudaMemcpyHostToDevice, st);
   if (e == cudaSuccess)
-    e = launch_tonemap(ctx->tm_in.ptr, n, y_mid, ctx->partials.ptr, nb, ctx->exposure,
+    e = launch_tonemap(ctx->tm_in.ptr, n, y_mid, ctx->partials.ptr, nb,
                        out_tonemapped ? ctx->tm_out.ptr : nullptr, out_rgb24 ? ctx->tm_24.ptr : nullptr, st);
   if (e == cudaSuccess && out_tonemapped)
     e = cudaMemcpyAsync(out_tonemapped, ctx->tm_out.ptr, 3 * n * sizeof(float), cudaMemcpyDeviceToHost, st);

@@ -312,7 +312,6 @@ cudaError_t launch_adjoint_k(const DevScene& S, const RenderArgs& a, WaveState* 
 constexpr uint32_t kTonemapMaxPartials = 148 * 8;
 uint32_t tonemap_partials_needed(uint64_t n_pixels);
 cudaError_t launch_tonemap(const float* d_rgb, uint64_t n_pixels, float y_mid, double* d_partials,
-                           uint32_t n_partials, float* d_exposure, float* d_out_tm,
-                           uint8_t* d_out24, cudaStream_t st);
+                           uint32_t n_partials, float* d_out_tm, uint8_t* d_out24, cudaStream_t st);
 
 }  // namespace lgpu

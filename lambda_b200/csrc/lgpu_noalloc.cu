@@ -4,8 +4,7 @@
 //
 // The tone map's scratch is the per-block partial sums of log-luminance
 // (at most kTonemapMaxPartials doubles for any image, the reduction is
-// grid-strided) and the exposure (one float).  Both live in
-// g_tonemap_scratch; host code gets its device address once per device with
+// grid-strided).  They live in g_tonemap_scratch; host code gets its device address once per device with
 // cudaGetSymbolAddress (the symbol itself is only a host-side stand-in) and
 // passes that address to the same kernels lgpu_tonemap launches.
 #include <cuda_runtime.h>
@@ -19,7 +18,7 @@ namespace {
 
 constexpr uint32_t kPartials = lgpu::kTonemapMaxPartials;
 constexpr size_t kScratchDoubles = LGPU_NOALLOC_SCRATCH_BYTES / sizeof(double);
-static_assert(kScratchDoubles >= kPartials + 1, "partials + the exposure slot");
+static_assert(kScratchDoubles >= kPartials, "the partial sums");
 
 static __device__ __align__(256) double g_tonemap_scratch[kScratchDoubles];
 
@@ -59,9 +58,7 @@ extern "C" int lgpu_tonemap_noalloc(const float* d_linrgb, uint64_t w, uint64_t 
   int const rc = scratch_address(&scratch);
   if (rc != LGPU_OK) return rc;
   cudaStream_t const st = static_cast<cudaStream_t>(stream);
-  float* exposure = reinterpret_cast<float*>(scratch + kPartials);
-  cudaError_t e = lgpu::launch_tonemap(d_linrgb, n, y_mid, scratch, kPartials, exposure, d_out_tonemapped,
-                                       d_out_rgb24, st);
+  cudaError_t e = lgpu::launch_tonemap(d_linrgb, n, y_mid, scratch, kPartials, d_out_tonemapped, d_out_rgb24, st);
   if (e == cudaSuccess) e = cudaStreamSynchronize(st);
   return e == cudaSuccess ? LGPU_OK : LGPU_ERR_CUDA;
 }
