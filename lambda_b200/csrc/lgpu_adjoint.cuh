@@ -17,7 +17,9 @@
 //   replay  the same paths again from their random streams (no shadow rays:
 //           visibility comes from the bits), starting from L and subtracting
 //           each vertex's contribution to get L_after_v, accumulating
-//           dL/dπ · dLoss/dL into the gradients.
+//           dL/dπ · dLoss/dL into the gradients.  Where they fit in memory
+//           the primal pass also records the vertices' hits, and the replay
+//           traces no rays at all.
 // Parameters: the bins of Lambertian albedo spectra and of thin-film IOR
 // spectra, thin-film thickness, and the exponent α of Blinn and thin-film
 // lobes.
@@ -27,51 +29,50 @@
 
 namespace lgpu {
 
-// ---- forward-mode derivatives of thinfilm::BRDFcosθ ------------------------------
+// ---- derivatives of thinfilm::BRDFcosθ --------------------------------------------
 
-// value and derivatives along two directions (film IOR n1, thickness d)
-struct Dual2 {
-  float v, a, b;
+// thinfilm_k (lgpu_path.cuh, cg.hpp:1001-1051), by the same operations, with
+// its derivatives with respect to the film IOR n1 and the thickness d.  With
+// q = sqrt(1 - 1/n1²), c = 1 - cos_i², φ = 4π n1 d q c / λ, and a, b the
+// difference and sum of the IORs at an interface (R0 = a²/b²):
+//     ∂φ/∂n1 = 4π d c / (λ q)    (n1 q = sqrt(n1² - 1)),   ∂φ/∂d = φ / d,
+//     ∂R0_01/∂n1 = -4 (1 - n1) / (1 + n1)³,   ∂R0_12/∂n1 = 4 (n1 - n2) n2 / (n1 + n2)³.
+// About 11 divisions where forward-mode dual numbers took 35, at the same
+// error (2-norm over 400,000 random films against double precision: ∂n1
+// 7.299e-3 with both, ∂d 9.416e-3; the rounding of φ makes it).
+struct FilmGrad {
+  float v, dn, dd;
 };
-__device__ __forceinline__ Dual2 dc(float x) { return Dual2{x, 0.f, 0.f}; }
-__device__ __forceinline__ Dual2 operator+(Dual2 x, Dual2 y) { return Dual2{x.v + y.v, x.a + y.a, x.b + y.b}; }
-__device__ __forceinline__ Dual2 operator-(Dual2 x, Dual2 y) { return Dual2{x.v - y.v, x.a - y.a, x.b - y.b}; }
-__device__ __forceinline__ Dual2 operator*(Dual2 x, Dual2 y) {
-  return Dual2{x.v * y.v, x.a * y.v + x.v * y.a, x.b * y.v + x.v * y.b};
-}
-__device__ __forceinline__ Dual2 operator/(Dual2 x, Dual2 y) {
-  float const q = x.v / y.v;
-  return Dual2{q, (x.a - q * y.a) / y.v, (x.b - q * y.b) / y.v};
-}
-__device__ __forceinline__ Dual2 dsqrt(Dual2 x) {
-  float const r = sqrtf(x.v);
-  float const h = r > 0.f ? 0.5f / r : 0.f;
-  return Dual2{r, x.a * h, x.b * h};
-}
-__device__ __forceinline__ Dual2 dcos(Dual2 x) {
-  float s, c;
-  sincosf(x.v, &s, &c);
-  return Dual2{c, -s * x.a, -s * x.b};
-}
-
-// thinfilm_k (lgpu_path.cuh, cg.hpp:1001-1051) with its value's derivatives
-// with respect to the film IOR n1 (.a) and the thickness d (.b)
-__device__ __forceinline__ Dual2 thinfilm_dual(float n1v, float n2v, float dv, float alpha, float l, float cos_i,
-                                               float pow5, float pow_hn) {
-  Dual2 const n1{n1v, 1.f, 0.f}, n2 = dc(n2v), d{dv, 0.f, 1.f};
-  Dual2 const one = dc(1.f);
-  Dual2 const n01 = one / n1;
-  Dual2 const cos_l = dsqrt(one - n01 * n01) * dc(1.f - cos_i * cos_i);
-  Dual2 const cos_d = dcos(dc(4.f * kPi) * n1 * d * cos_l / dc(l));
-  Dual2 const a01 = one - n1, b01 = one + n1;
-  Dual2 const R0_01 = a01 * a01 / (b01 * b01);
-  Dual2 const a12 = n1 - n2, b12 = n1 + n2;
-  Dual2 const R0_12 = a12 * a12 / (b12 * b12);
-  Dual2 const R01 = R0_01 + (one - R0_01) * dc(pow5);
-  Dual2 const R12 = R0_12 + (one - R0_12) * dc(pow5);
-  Dual2 const Ravg = dc(2.f) * dsqrt(R01 * R12);
-  Dual2 const Rt = (R01 + R12 + Ravg * cos_d) / (one + R01 * R12 + Ravg * cos_d);
-  return dc((alpha + 2.f) * 0.125f * kInvPi * pow_hn) * Rt;
+__device__ __forceinline__ FilmGrad thinfilm_grad(float n1, float n2, float d, float alpha, float l, float cos_i,
+                                                  float pow5, float pow_hn) {
+  float const n01 = 1.f / n1;
+  float const q = sqrtf(1.f - n01 * n01), c = 1.f - cos_i * cos_i;
+  float const cos_l = q * c;
+  float sn, cs;
+  sincosf(4.f * kPi * n1 * d * cos_l / l, &sn, &cs);
+  float const a01 = (1.f - n1), b01 = (1.f + n1);
+  float const R0_01 = a01 * a01 / (b01 * b01);
+  float const a12 = (n1 - n2), b12 = (n1 + n2);
+  float const R0_12 = a12 * a12 / (b12 * b12);
+  float const R01 = R0_01 + (1.f - R0_01) * pow5;
+  float const R12 = R0_12 + (1.f - R0_12) * pow5;
+  float const P = R01 * R12, root = sqrtf(P), Ravg = 2.f * root;
+  float const den = 1.f + P + Ravg * cs;
+  float const Rt = (R01 + R12 + Ravg * cs) / den;
+  // derivatives
+  float const k4 = 4.f * kPi / l, i01 = 1.f / b01, i12 = 1.f / b12, iden = 1.f / den;
+  float const phi_n = q > 0.f ? k4 * d * c / q : 0.f, phi_d = k4 * n1 * cos_l;
+  float const keep = 1.f - pow5;
+  float const R01n = -4.f * a01 * (i01 * i01 * i01) * keep, R12n = 4.f * a12 * n2 * (i12 * i12 * i12) * keep;
+  float const Pn = R01n * R12 + R01 * R12n;
+  float const avg_n = root > 0.f ? Pn / root : 0.f;
+  float const Xn = avg_n * cs - Ravg * sn * phi_n, Xd = -Ravg * sn * phi_d;
+  float const s = (alpha + 2.f) * 0.125f * kInvPi * pow_hn;
+  FilmGrad f;
+  f.v = (alpha + 2.f) * 0.125f * kInvPi * Rt * pow_hn;
+  f.dn = s * (((R01n + R12n + Xn) - Rt * (Pn + Xn)) * iden);
+  f.dd = s * (Xd * (1.f - Rt) * iden);
+  return f;
 }
 
 // ---- accumulation ---------------------------------------------------------------
@@ -100,67 +101,21 @@ __device__ __forceinline__ float dlog_lobe_dalpha(float alpha, float c, float ln
   return c > 0.f ? 1.f / (alpha + 2.f) + lnhn : 0.f;
 }
 
-// v * d BxDFcosθ(light dir) / dπ for the NEE term (bsdf_k's cases)
-__device__ __forceinline__ void grad_bsdf(const DevScene& S, const DevMaterial& m, uint32_t mat,
-                                          const BsdfScalars& r, float x, float l, bool front, float v,
-                                          const AdjointArgs& g, float& g_d, float& g_alpha) {
-  switch (r.kind) {
-    case 1:
-      spec_grad(S, g.g_spec, m.spectrum[0], x, v * kInvPi * r.a);
-      break;
-    case 2:
-    case 3: {
-      float const ior = spec_at(S, m.spectrum[4], x);
-      float const eta = front ? 1.f / ior : ior;
-      float const F0 = schlick_F0(eta);
-      float const F = F0 + (1.f - F0) * r.b;
-      float const gl = (m.alpha + 2.f) * 0.125f * kInvPi * r.c;
-      float const spec = r.kind == 2 ? (spec_at(S, m.spectrum[1], x) + F * spec_at(S, m.spectrum[2], x)) * gl
-                                     : spec_at(S, m.spectrum[2], x) * (1.f - F) * gl;
-      g_alpha += v * spec * dlog_lobe_dalpha(m.alpha, r.c, r.lnhn);
-      break;
-    }
-    case 4: {
-      Dual2 const f = thinfilm_dual(spec_at(S, m.spectrum[0], x), spec_at(S, m.spectrum[1], x), m.d, m.alpha, l,
-                                    r.a, r.b, r.c);
-      spec_grad(S, g.g_spec, m.spectrum[0], x, v * f.a);
-      g_d += v * f.b;
-      g_alpha += v * f.v * dlog_lobe_dalpha(m.alpha, r.c, r.lnhn);
-      break;
-    }
-  }
-  (void)mat;
+// v * d BxDFcosθ(light dir) / dα for the NEE term of a Blinn lobe (bsdf_k's
+// cases 2 and 3)
+__device__ __forceinline__ float grad_blinn(const DevScene& S, const DevMaterial& m, const BsdfScalars& r, float x,
+                                            bool front, float v) {
+  float const ior = spec_at(S, m.spectrum[4], x);
+  float const eta = front ? 1.f / ior : ior;
+  float const F0 = schlick_F0(eta);
+  float const F = F0 + (1.f - F0) * r.b;
+  float const gl = (m.alpha + 2.f) * 0.125f * kInvPi * r.c;
+  float const spec = r.kind == 2 ? (spec_at(S, m.spectrum[1], x) + F * spec_at(S, m.spectrum[2], x)) * gl
+                                 : spec_at(S, m.spectrum[2], x) * (1.f - F) * gl;
+  return v * spec * dlog_lobe_dalpha(m.alpha, r.c, r.lnhn);
 }
 
-// u * d ln f / dπ for the material sample's BSDF value f = mat_mult_k
-// (u = dLoss/dL * L_after at this wavelength)
-__device__ __forceinline__ void grad_mult(const DevScene& S, const DevMaterial& m, const MatSample& ms, float x,
-                                          float l, float f, float u, const AdjointArgs& g, float& g_d,
-                                          float& g_alpha) {
-  if (f == 0.f || u == 0.f) return;
-  switch (ms.lobe) {
-    case 1:
-      if (m.type == LGPU_MAT_LAMBERTIAN) {
-        float const alb = spec_at(S, m.spectrum[0], x);
-        if (alb != 0.f) spec_grad(S, g.g_spec, m.spectrum[0], x, u / alb);
-      }
-      break;
-    case 2:
-    case 3:
-      g_alpha += u * dlog_lobe_dalpha(m.alpha, ms.c, ms.lnhn);
-      break;
-    case 4: {
-      Dual2 const t = thinfilm_dual(spec_at(S, m.spectrum[0], x), spec_at(S, m.spectrum[1], x), m.d, m.alpha, l,
-                                    ms.a, ms.b, ms.c);
-      if (t.v != 0.f) {
-        spec_grad(S, g.g_spec, m.spectrum[0], x, u * t.a / t.v);
-        g_d += u * t.b / t.v;
-      }
-      g_alpha += u * dlog_lobe_dalpha(m.alpha, ms.c, ms.lnhn);
-      break;
-    }
-  }
-}
+__device__ __forceinline__ float finite_or_zero(float x) { return isfinite(x) ? x : 0.f; }
 
 namespace {
 
@@ -231,12 +186,19 @@ __global__ void __launch_bounds__(256) wf_replay_generate(OneJob jobs, WaveState
 }
 
 // One vertex of the replay: the same random decisions as wf_shade, the
-// visibility recorded by the primal pass, gradients accumulated.
-template <int K>
-// 10 blocks of 128 per SM: like the forward shading, latency-bound, so more
-// warps beat fewer spills (5 blocks at 89 registers made the adjoint 5 %
-// slower).
-__global__ void __launch_bounds__(128, 10) wf_shade_adjoint(OneJob jobs, WaveState w, AdjointArgs g) {
+// visibility recorded by the primal pass, gradients accumulated.  Three
+// launches by material like wf_shade's (MT: Lambertian and the rest, which
+// also lists the others; Blinn; thin film).
+//
+// Bound by issue and by instruction fetch (5 of 16 stalls in one launch for
+// all materials, with the gradient code of each in every block).  64x64
+// thin-film tiles under 64 spheres, 512x512, 32 spp: one launch with
+// forward-mode dual numbers 18.8 ms, closed-form thin-film derivatives 10.7
+// ms, three launches 6.6 ms (4 blocks of 256 per SM; 3
+// and 5: +5 %); the bins' atomics are no bound (without
+// them 18.4 of the 18.8 ms).
+template <int K, int MT>
+__global__ void __launch_bounds__(kMaxShadeBlock, 4) wf_shade_adjoint(OneJob jobs, WaveState w, AdjointArgs g) {
   uint32_t const n = *w.n_in;
   uint32_t const cap = w.cap;
   const DevScene& S = jobs.S;
@@ -245,9 +207,26 @@ __global__ void __launch_bounds__(128, 10) wf_shade_adjoint(OneJob jobs, WaveSta
   PathBuf const& out = w.out;
   float const omega = S.lambda_sup - S.lambda_inf;
   float const step = omega / float(K);
-  for (uint32_t base = blockIdx.x * blockDim.x; base < n; base += gridDim.x * blockDim.x) {
-    uint32_t const i = material_order(jobs, w, base, n);
-    bool const live = i < n;
+  constexpr bool kList = MT == LGPU_MAT_BLINN || MT == LGPU_MAT_THINFILM;
+  uint32_t const n_loop = kList ? w.ctl[MT == LGPU_MAT_BLINN ? kCtlListB : kCtlListT] : n;
+  for (uint32_t base = blockIdx.x * blockDim.x; base < n_loop; base += gridDim.x * blockDim.x) {
+    uint32_t group = 1u + MT, i;
+    if (kList) {
+      uint32_t const j = base + threadIdx.x;
+      i = j < n_loop ? w.shade_list[MT == LGPU_MAT_BLINN ? j : cap - 1u - j] : UINT32_MAX;
+    } else {
+      i = material_order(jobs, w, base, n, &group, [&](uint32_t q) {
+        return w.v_obj ? w.v_obj[size_t(__float_as_uint(in.rb[q].w)) * w.v_items + in.rc[q].z] : w.hobj[q];
+      });
+      list_material_groups(w, i, group);
+    }
+    bool const live = i < n && shade_group<MT>(group);
+    auto material = [&](uint32_t idx) {
+      DevMaterial x = S.mats[idx];
+      if (kList) x.type = MT;
+      if (!kList && (x.type == LGPU_MAT_BLINN || x.type == LGPU_MAT_THINFILM)) x.type = LGPU_MAT_MICROFACET;
+      return x;
+    };
     bool cont = false, scatter = false, visible = false;
     f3 np = f3{0.f, 0.f, 0.f}, nd = f3{0.f, 0.f, 1.f};
     float lis_scale = 0.f, m_scale = 0.f, hero = 0.f;
@@ -265,9 +244,10 @@ __global__ void __launch_bounds__(128, 10) wf_shade_adjoint(OneJob jobs, WaveSta
       hero = rb.z;
       depth = __float_as_uint(rb.w);
       item = rc.z;
-      uint32_t const obj = w.hobj[i];
+      size_t const v_at = size_t(depth) * w.v_items + item;
+      uint32_t const obj = w.v_obj ? w.v_obj[v_at] : w.hobj[i];
       if (obj != UINT32_MAX) {
-        HitRec const h = load_hit(w, i, obj);
+        HitRec const h = w.v_obj ? load_hit(w.v_hita, w.v_hitb, v_at, obj) : load_hit(w.hita, w.hitb, i, obj);
         Ray const r = make_ray(in.ra[i], rb);
         HitInfo const H = finalize_hit(S, r, h);
         f3 const un = fnorm(r.u);
@@ -275,7 +255,7 @@ __global__ void __launch_bounds__(128, 10) wf_shade_adjoint(OneJob jobs, WaveSta
         f3 const nn = H.front ? H.F.z : neg3(H.F.z);
         mat = H.mat;
         front = H.front;
-        const DevMaterial& m = S.mats[mat];
+        DevMaterial const m = material(mat);
         // an emitter ends the path; its radiance is not a parameter
         if (m.type != LGPU_MAT_EMITTER && m.type != LGPU_MAT_DIREMITTER && depth <= a.max_scatter) {
           scatter = true;
@@ -324,9 +304,24 @@ __global__ void __launch_bounds__(128, 10) wf_shade_adjoint(OneJob jobs, WaveSta
         }
       }
     }
+    // what this launch's materials leave of the BSDF cases and lobes
+    if (MT == LGPU_MAT_LAMBERTIAN) {
+      bl.kind = bl.kind ? 1 : 0;
+      ms.lobe = ms.lobe ? 1 : 0;
+    } else if (MT == LGPU_MAT_BLINN) {
+      bl.kind = bl.kind == 2 ? 2 : 3;
+    } else {
+      bl.kind = bl.kind ? 4 : 0;
+      ms.lobe = ms.lobe ? 4 : 0;
+    }
     uint32_t const o_pos = warp_append(w.n_out, cont);
     if (!scatter) continue;
-    const DevMaterial& m = S.mats[mat];
+    if (cont) {
+      out.ra[o_pos] = make_float4(np.x, np.y, np.z, nd.x);
+      out.rb[o_pos] = make_float4(nd.y, nd.z, hero, __uint_as_float(depth + 1));
+      out.rc[o_pos] = make_uint4(uint32_t(rng), uint32_t(rng >> 32), item, kNoShadow);
+    }
+    DevMaterial const m = material(mat);
     const lgpu_light& L = S.lights[light];
     float g_d = 0.f, g_alpha = 0.f;
     float4 bt = make_float4(0.f, 0.f, 0.f, 0.f), gws = bt, rems = bt;
@@ -342,20 +337,61 @@ __global__ void __launch_bounds__(128, 10) wf_shade_adjoint(OneJob jobs, WaveSta
       float const x = lam_coord(S, l);
       float const gw = gws.x;
       float b = bt.x, rem = rems.x;
+      // the spectrum the material's gradient goes to (Lambertian albedo or
+      // film IOR): the light sample's and the material sample's part together
+      float g_bin = 0.f;
+      float n1 = 0.f, n2 = 0.f;
+      if (m.type == LGPU_MAT_THINFILM) {
+        n1 = spec_at(S, m.spectrum[0], x);
+        n2 = spec_at(S, m.spectrum[1], x);
+      }
       if (visible && lis_scale != 0.f) {
-        float const coef = bsdf_k(S, m, bl, x, l, front);
         float const rad = spec_at(S, L.spectrum, x);
-        grad_bsdf(S, m, mat, bl, x, l, front, gw * b * rad * lis_scale, g, g_d, g_alpha);
+        float const v = gw * b * rad * lis_scale;
+        float coef;
+        if (bl.kind == 4) {
+          FilmGrad const f = thinfilm_grad(n1, n2, m.d, m.alpha, l, bl.a, bl.b, bl.c);
+          coef = f.v;
+          g_bin += finite_or_zero(v * f.dn);
+          g_d += v * f.dd;
+          g_alpha += v * f.v * dlog_lobe_dalpha(m.alpha, bl.c, bl.lnhn);
+        } else {
+          coef = bsdf_k(S, m, bl, x, l, front);
+          if (bl.kind == 1) g_bin += finite_or_zero(v * kInvPi * bl.a);
+          else if (bl.kind != 0) g_alpha += grad_blinn(S, m, bl, x, front, v);
+        }
         float const nee = b * (rad * coef * lis_scale);
         g_alpha += gw * nee * dlw_L;
         rem -= nee;
       }
       if (cont) {
-        float const f = mat_mult_k(S, m, ms, x, l, front);
-        grad_mult(S, m, ms, x, l, f, gw * rem, g, g_d, g_alpha);
-        g_alpha += gw * rem * dlw_mat;
+        // u * d ln f / dπ of the material sample's BSDF value f
+        float const u = gw * rem;
+        float f;
+        if (ms.lobe == 4) {
+          FilmGrad const t = thinfilm_grad(n1, n2, m.d, m.alpha, l, ms.a, ms.b, ms.c);
+          f = t.v;
+          if (f != 0.f && u != 0.f) {
+            float const uf = u / f;
+            g_bin += finite_or_zero(uf * t.dn);
+            g_d += uf * t.dd;
+            g_alpha += u * dlog_lobe_dalpha(m.alpha, ms.c, ms.lnhn);
+          }
+        } else {
+          f = mat_mult_k(S, m, ms, x, l, front);
+          if (f != 0.f && u != 0.f) {
+            if (ms.lobe == 1) {
+              float const alb = m.type == LGPU_MAT_LAMBERTIAN ? spec_at(S, m.spectrum[0], x) : 0.f;
+              if (alb != 0.f) g_bin += finite_or_zero(u / alb);
+            } else {
+              g_alpha += u * dlog_lobe_dalpha(m.alpha, ms.c, ms.lnhn);
+            }
+          }
+        }
+        g_alpha += u * dlw_mat;
         b = b * (f * m_scale);
       }
+      if (g_bin != 0.f) spec_grad(S, g.g_spec, m.spectrum[0], x, g_bin);
       // the words turn by one wavelength (see wf_shade)
       bt = make_float4(bt.y, bt.z, bt.w, b);
       gws = make_float4(gws.y, gws.z, gws.w, gw);
@@ -368,11 +404,6 @@ __global__ void __launch_bounds__(128, 10) wf_shade_adjoint(OneJob jobs, WaveSta
     }
     if (g_d != 0.f && isfinite(g_d)) atomicAdd(g.g_mat + 4 * size_t(mat), g_d);
     if (g_alpha != 0.f && isfinite(g_alpha)) atomicAdd(g.g_mat + 4 * size_t(mat) + 1, g_alpha);
-    if (cont) {
-      out.ra[o_pos] = make_float4(np.x, np.y, np.z, nd.x);
-      out.rb[o_pos] = make_float4(nd.y, nd.z, hero, __uint_as_float(depth + 1));
-      out.rc[o_pos] = make_uint4(uint32_t(rng), uint32_t(rng >> 32), item, kNoShadow);
-    }
   }
 }
 
@@ -393,15 +424,21 @@ cudaError_t replay_chunk(const OneJob& jobs, WaveState& w, uint64_t c0, uint32_t
   return run_iterations(w, total, st, run, [&](const WaveState& wi) {
     wf_plan<<<1, 1, 0, st>>>(wi, total);
     wf_replay_generate<K><<<sms * gen_per_sm, 256, 0, st>>>(jobs, wi, g);
-    run->begin(0, st);
-    launch_closest<K>(jobs, wi, gr, linear, c_closest, st);
-    run->end(0, st);
+    if (!wi.v_obj) {
+      run->begin(0, st);
+      launch_closest<K>(jobs, wi, gr, linear, c_closest, st);
+      run->end(0, st);
+      run->total += closest_launches(jobs, linear);
+    }
     run->begin(2, st);
     // one block per queue chunk (see wave_chunk)
-    wf_shade_adjoint<K><<<(wi.cap + 127) / 128, 128, 0, st>>>(jobs, wi, g);
+    uint32_t const sg = (wi.cap + gr.shade_block - 1) / gr.shade_block;
+    wf_shade_adjoint<K, LGPU_MAT_LAMBERTIAN><<<sg, gr.shade_block, 0, st>>>(jobs, wi, g);
+    wf_shade_adjoint<K, LGPU_MAT_BLINN><<<sg, gr.shade_block, 0, st>>>(jobs, wi, g);
+    wf_shade_adjoint<K, LGPU_MAT_THINFILM><<<sg, gr.shade_block, 0, st>>>(jobs, wi, g);
     run->end(2, st);
-    // plan, generate, shade
-    run->total += 3 + closest_launches(jobs, linear);
+    // plan, generate, shade (3)
+    run->total += 5;
   });
 }
 

@@ -88,6 +88,13 @@ struct WaveState {
   uint64_t* vis;       // per work item: bit v set = the shadow ray of vertex v reached its light
   uint32_t* s_item;    // cap: work item of each shadow ray
   uint32_t* s_depth;   // cap: its vertex
+  // the hits of the primal pass's scattering vertices, vertex v of work item
+  // q at v*v_items + q (obj, hita, hitb as above; obj UINT32_MAX where the
+  // path ends), so that the replay traces no rays; nullptr: it does
+  uint32_t* v_obj;
+  float4* v_hita;
+  float4* v_hitb;
+  uint64_t v_items;    // work items of a chunk
 };
 
 struct RenderArgs {

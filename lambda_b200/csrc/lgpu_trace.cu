@@ -46,7 +46,7 @@ __global__ void __launch_bounds__(128) trace_store(DevScene S, WaveState w, uint
   uint32_t const obj = w.hobj[i];
   lgpu_hit o;
   if (obj != UINT32_MAX) {
-    HitInfo const H = finalize_hit(S, load_ray(w.in.ra, w.in.rb, i), load_hit(w, i, obj));
+    HitInfo const H = finalize_hit(S, load_ray(w.in.ra, w.in.rb, i), load_hit(w.hita, w.hitb, i, obj));
     o.t = H.z;
     o.obj = H.obj;
     o.face = H.face;

@@ -67,8 +67,8 @@ __device__ __forceinline__ void store_hit(const WaveState& w, uint32_t p, const 
   if (h.obj != UINT32_MAX) store_hit_point(w, p, h.face, h.b0, h.b1, h.b2, h.pl, h.z);
 }
 // the record of a path that hit object `obj`
-__device__ __forceinline__ HitRec load_hit(const WaveState& w, uint32_t p, uint32_t obj) {
-  float4 const a = w.hita[p], b = w.hitb[p];
+__device__ __forceinline__ HitRec load_hit(const float4* hita, const float4* hitb, size_t p, uint32_t obj) {
+  float4 const a = hita[p], b = hitb[p];
   HitRec h;
   h.obj = obj;
   h.z = b.w;
@@ -561,9 +561,10 @@ __global__ void __launch_bounds__(128) wf_trace_fallback(J jobs, WaveState w, De
 // each thread's rank within its group.  Returns the entry for this thread.
 constexpr int kSortGroups = 8;
 
-template <class J>
+// obj_of(q) is the object that entry q hit (UINT32_MAX: none).
+template <class J, class O>
 __device__ __forceinline__ uint32_t material_order(const J& jobs, const WaveState& w, uint32_t base, uint32_t n,
-                                                   uint32_t* group = nullptr) {
+                                                   uint32_t* group, O obj_of) {
   __shared__ uint32_t counts[kSortGroups][kMaxShadeBlock / 32];
   __shared__ uint16_t perm[kMaxShadeBlock];
   __shared__ uint8_t groups[kMaxShadeBlock];
@@ -571,7 +572,7 @@ __device__ __forceinline__ uint32_t material_order(const J& jobs, const WaveStat
   uint32_t const q = base + t;
   uint32_t key = kSortGroups - 1;
   if (q < n) {
-    uint32_t const obj = w.hobj[q];
+    uint32_t const obj = obj_of(q);
     if (obj == UINT32_MAX) {
       key = 0;
     } else {
@@ -596,7 +597,7 @@ __device__ __forceinline__ uint32_t material_order(const J& jobs, const WaveStat
   groups[pos] = uint8_t(key);
   __syncthreads();
   uint32_t const r = base + perm[t];
-  if (group) *group = groups[t];
+  *group = groups[t];
   __syncthreads();  // counts and perm are reused by the block's next chunk
   return r;
 }
@@ -672,7 +673,7 @@ __global__ void __launch_bounds__(kMaxShadeBlock, 4) wf_shade(J jobs, WaveState 
       i = j < n_loop ? w.shade_list[MT == LGPU_MAT_BLINN ? j : cap - 1u - j] : UINT32_MAX;
       group = 1u + MT;
     } else {
-      i = material_order(jobs, w, base, n, &group);
+      i = material_order(jobs, w, base, n, &group, [&](uint32_t q) { return w.hobj[q]; });
       if (MT == LGPU_MAT_LAMBERTIAN) list_material_groups(w, i, group);
     }
     bool const live = i < n && shade_group<MT>(group);
@@ -713,8 +714,10 @@ __global__ void __launch_bounds__(kMaxShadeBlock, 4) wf_shade(J jobs, WaveState 
       item = rc.z;
       prev_s = rc.w;
       uint32_t const obj = w.hobj[i];
+      size_t const v_at = size_t(depth) * w.v_items + item;
+      if (w.v_obj) w.v_obj[v_at] = UINT32_MAX;
       if (obj != UINT32_MAX) {
-        HitRec const h = load_hit(w, i, obj);
+        HitRec const h = load_hit(w.hita, w.hitb, i, obj);
         Ray const r = make_ray(in.ra[i], rb);
         HitInfo const H = finalize_hit(S, r, h);
         f3 const un = fnorm(r.u);
@@ -731,6 +734,11 @@ __global__ void __launch_bounds__(kMaxShadeBlock, 4) wf_shade(J jobs, WaveState 
           }
         } else if (depth <= a.max_scatter) {
           kind = kScatter;
+          if (w.v_obj) {
+            w.v_obj[v_at] = obj;
+            w.v_hita[v_at] = make_float4(__uint_as_float(h.face), h.b0, h.b1, h.b2);
+            w.v_hitb[v_at] = make_float4(h.pl.x, h.pl.y, h.pl.z, h.z);
+          }
           rng = (uint64_t(rc.y) << 32) | rc.x;
           light = uint32_t(lgpu_u64(&rng) % uint64_t(S.n_lights));
           float const prob_l = 1.f / float(S.n_lights);
