@@ -421,9 +421,9 @@ cudaError_t replay_chunk(const OneJob& jobs, WaveState& w, uint64_t c0, uint32_t
   w.c0 = c0;
   wf_stream_init<<<1, 32, 0, st>>>(w);
   run->total++;
-  return run_iterations(w, total, st, run, [&](const WaveState& wi) {
+  return run_iterations(w, total, jobs.max_scatter(), st, run, [&](const WaveState& wi, bool generate) {
     wf_plan<<<1, 1, 0, st>>>(wi, total);
-    wf_replay_generate<K><<<sms * gen_per_sm, 256, 0, st>>>(jobs, wi, g);
+    if (generate) wf_replay_generate<K><<<sms * gen_per_sm, 256, 0, st>>>(jobs, wi, g);
     if (!wi.v_obj) {
       run->begin(0, st);
       launch_closest<K>(jobs, wi, gr, linear, c_closest, st);
@@ -434,11 +434,12 @@ cudaError_t replay_chunk(const OneJob& jobs, WaveState& w, uint64_t c0, uint32_t
     // one block per queue chunk (see wave_chunk)
     uint32_t const sg = (wi.cap + gr.shade_block - 1) / gr.shade_block;
     wf_shade_adjoint<K, LGPU_MAT_LAMBERTIAN><<<sg, gr.shade_block, 0, st>>>(jobs, wi, g);
-    wf_shade_adjoint<K, LGPU_MAT_BLINN><<<sg, gr.shade_block, 0, st>>>(jobs, wi, g);
-    wf_shade_adjoint<K, LGPU_MAT_THINFILM><<<sg, gr.shade_block, 0, st>>>(jobs, wi, g);
+    bool const blinn = jobs.has_material(LGPU_MAT_BLINN), film = jobs.has_material(LGPU_MAT_THINFILM);
+    if (blinn) wf_shade_adjoint<K, LGPU_MAT_BLINN><<<sg, gr.shade_block, 0, st>>>(jobs, wi, g);
+    if (film) wf_shade_adjoint<K, LGPU_MAT_THINFILM><<<sg, gr.shade_block, 0, st>>>(jobs, wi, g);
     run->end(2, st);
-    // plan, generate, shade (3)
-    run->total += 5;
+    // plan, shade
+    run->total += 2 + (generate ? 1 : 0) + (blinn ? 1 : 0) + (film ? 1 : 0);
   });
 }
 
@@ -455,7 +456,7 @@ cudaError_t launch_adjoint_k(const DevScene& S, const RenderArgs& a, WaveState* 
   cudaError_t e = cudaMemsetAsync(w.film, 0, sizeof(float) * 3 * size_t(w.npix), st);
   for (uint64_t c0 = 0; c0 < n_items && e == cudaSuccess; c0 += chunk_items) {
     uint32_t const total = uint32_t(n_items - c0 < chunk_items ? n_items - c0 : chunk_items);
-    e = wave_chunk<K>(jobs, w, c0, total, linear, d_cnt, st, run);
+    e = wave_chunk<K, true>(jobs, w, c0, total, linear, d_cnt, st, run);
     if (e == cudaSuccess) e = replay_chunk<K>(jobs, w, c0, total, linear, g, d_cnt, st, run);
   }
   if (e == cudaSuccess && d_img) e = finalize_film<K>(jobs, w, st, run);

@@ -494,11 +494,13 @@ int batch_impl(lgpu_ctx* ctx, const lgpu_job* jobs, uint32_t n, float* const* d_
   std::vector<uint64_t> items(n + 1);
   std::vector<uint32_t> pixels(n + 1);
   uint64_t g = 0, px = 0;
-  uint32_t max_objects = 0;
+  JobTable table{};
   for (uint32_t k = 0; k < n; k++) {
     DevJob& d = hj[k];
     d.S = ctx->slots[jobs[k].scene].S;
-    max_objects = std::max(max_objects, d.S.n_objects);
+    table.objects = std::max(table.objects, d.S.n_objects);
+    table.mat_types |= d.S.mat_types;
+    table.max_bounces = std::max(table.max_bounces, jobs[k].params.max_scatterings);
     d.a = render_args(&jobs[k].params, d.S);
     uint32_t th = 0;
     job_rect(jobs[k], d.S.cam, d.col0, d.row0, d.tile_w, th);
@@ -530,14 +532,17 @@ int batch_impl(lgpu_ctx* ctx, const lgpu_job* jobs, uint32_t n, float* const* d_
     e = cudaMemcpyAsync(ctx->job_pixels.ptr, pixels.data(), (n + 1) * sizeof(uint32_t), cudaMemcpyHostToDevice,
                         st);
   if (e != cudaSuccess) return cuda_fail(ctx, e, "batch tables");
+  table.d = ctx->jobs.ptr;
+  table.item_bases = ctx->job_items.ptr;
+  table.pix_bases = ctx->job_pixels.ptr;
+  table.n = n;
   WaveState ws{};
   if (int r = ensure_wave(ctx, uint32_t(px), g, chunk, true, ws)) return r;
   if (int r = prepare_launch(ctx, timing)) return r;
   e = ctx->keep_counters ? cudaSuccess : cudaMemsetAsync(ctx->counters, 0, 3 * sizeof(DevCounters), st);
   if (e == cudaSuccess) e = cudaEventRecord(ctx->ev0, st);
   if (e == cudaSuccess)
-    e = launch_batch(ctx->S.hero_k, ctx->jobs.ptr, ctx->job_items.ptr, ctx->job_pixels.ptr, n, max_objects, g, chunk,
-                     linear, &ws, ctx->counters, st, &ctx->launch);
+    e = launch_batch(ctx->S.hero_k, table, g, chunk, linear, &ws, ctx->counters, st, &ctx->launch);
   if (e == cudaSuccess) e = cudaEventRecord(ctx->ev1, st);
   // the host tables must outlive their asynchronous copies
   if (e == cudaSuccess) e = cudaStreamSynchronize(st);
@@ -597,6 +602,13 @@ bool batch_timing(const lgpu_job* jobs, uint32_t n) {
 // per-kernel timing applies to the wavefront kernels only
 bool timing_requested(const lgpu_render_params* p) {
   return (p->flags & LGPU_FLAG_KERNEL_TIMING) && !(p->flags & LGPU_FLAG_MEGAKERNEL);
+}
+
+// The material types a scene has, one bit each.
+uint32_t material_types(const std::vector<DevMaterial>& mats) {
+  uint32_t t = 0;
+  for (const DevMaterial& m : mats) t |= 1u << m.type;
+  return t;
 }
 
 // Lays out one scene on the host and copies it into a scene slot.
@@ -832,6 +844,7 @@ int upload_slot(lgpu_ctx* ctx, SceneSlot& sl, const lgpu_scene& scene_in) {
   S.shade = sl.shade.ptr;
   S.spectra = sl.spectra.ptr;
   S.mats = sl.mats.ptr;
+  S.mat_types = material_types(L.mats);
   S.lights = sl.lights.ptr;
   S.tlas_objects = sl.tlas_objects.ptr;
   S.n_objects = scene.n_objects;
@@ -994,6 +1007,7 @@ int lgpu_update_materials(lgpu_ctx* ctx, const lgpu_scene* scene) {
     e = cudaMemcpyAsync(sl.spectra.ptr, scene->spectra, sl.spectra.n * sizeof(float), cudaMemcpyHostToDevice, st);
   if (e == cudaSuccess) e = cudaStreamSynchronize(st);
   if (e != cudaSuccess) return cuda_fail(ctx, e, "material update");
+  ctx->S.mat_types = sl.S.mat_types = material_types(mats);
   return LGPU_OK;
 }
 

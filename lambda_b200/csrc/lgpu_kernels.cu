@@ -147,21 +147,13 @@ cudaError_t launch_render(const DevScene& S, const RenderArgs& a, WaveState* wav
   return cudaErrorInvalidValue;
 }
 
-cudaError_t launch_batch(uint32_t hero_k, const DevJob* d_jobs, const uint64_t* d_item_bases,
-                         const uint32_t* d_pix_bases, uint32_t n_jobs, uint32_t max_objects, uint64_t n_items,
-                         uint64_t chunk_items, bool linear, WaveState* wave, DevCounters* d_cnt,
-                         cudaStream_t st, WaveLaunch* run) {
-  if (n_jobs == 0 || n_items == 0) return cudaSuccess;
+cudaError_t launch_batch(uint32_t hero_k, const JobTable& jobs, uint64_t n_items, uint64_t chunk_items, bool linear,
+                         WaveState* wave, DevCounters* d_cnt, cudaStream_t st, WaveLaunch* run) {
+  if (jobs.n == 0 || n_items == 0) return cudaSuccess;
   switch (hero_k) {
-    case 4:
-      return launch_batch_k<4>(d_jobs, d_item_bases, d_pix_bases, n_jobs, max_objects, n_items, chunk_items, linear,
-                               wave, d_cnt, st, run);
-    case 8:
-      return launch_batch_k<8>(d_jobs, d_item_bases, d_pix_bases, n_jobs, max_objects, n_items, chunk_items, linear, wave,
-                               d_cnt, st, run);
-    case 16:
-      return launch_batch_k<16>(d_jobs, d_item_bases, d_pix_bases, n_jobs, max_objects, n_items, chunk_items, linear, wave,
-                                d_cnt, st, run);
+    case 4: return launch_batch_k<4>(jobs, n_items, chunk_items, linear, wave, d_cnt, st, run);
+    case 8: return launch_batch_k<8>(jobs, n_items, chunk_items, linear, wave, d_cnt, st, run);
+    case 16: return launch_batch_k<16>(jobs, n_items, chunk_items, linear, wave, d_cnt, st, run);
   }
   return cudaErrorInvalidValue;
 }

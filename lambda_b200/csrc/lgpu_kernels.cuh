@@ -210,6 +210,8 @@ struct OneJob {
   uint32_t npix;
   float* out;
   uint32_t max_objects() const { return S.n_objects; }
+  uint32_t max_scatter() const { return a.max_scatter; }
+  bool has_material(int type) const { return (S.mat_types >> type) & 1u; }
   __device__ __forceinline__ const DevScene& scene(uint32_t) const { return S; }
   __device__ __forceinline__ const RenderArgs& args(uint32_t) const { return a; }
   __device__ __forceinline__ uint32_t job_of_item(uint64_t) const { return 0; }
@@ -229,7 +231,11 @@ struct JobTable {
   const uint32_t* pix_bases;   // n + 1 entries
   uint32_t n;
   uint32_t objects;            // of the job's scene that has the most
+  uint32_t mat_types;          // of all the jobs' scenes (DevScene::mat_types)
+  uint32_t max_bounces;        // of all the jobs (RenderArgs::max_scatter)
   uint32_t max_objects() const { return objects; }
+  uint32_t max_scatter() const { return max_bounces; }
+  bool has_material(int type) const { return (mat_types >> type) & 1u; }
   __device__ __forceinline__ const DevScene& scene(uint32_t j) const { return d[j].S; }
   __device__ __forceinline__ const RenderArgs& args(uint32_t j) const { return d[j].a; }
   // the job whose range holds item g / pixel gp (binary search)
@@ -277,16 +283,13 @@ cudaError_t launch_trace_chunk(const DevScene& S, WaveState& w, const float* d_r
                                cudaStream_t st);
 
 // Batched render of the jobs of `table` (n jobs, n_items work items,
-// n_pix pixels in all; max_objects in the largest scene) with the wavefront
-// kernels.
-cudaError_t launch_batch(uint32_t hero_k, const DevJob* d_jobs, const uint64_t* d_item_bases,
-                         const uint32_t* d_pix_bases, uint32_t n_jobs, uint32_t max_objects, uint64_t n_items,
-                         uint64_t chunk_items, bool linear, WaveState* wave, DevCounters* d_cnt,
-                         cudaStream_t st, WaveLaunch* run);
+// n_pix pixels in all) with the wavefront kernels.
+struct JobTable;
+cudaError_t launch_batch(uint32_t hero_k, const JobTable& jobs, uint64_t n_items, uint64_t chunk_items, bool linear,
+                         WaveState* wave, DevCounters* d_cnt, cudaStream_t st, WaveLaunch* run);
 template <int K>
-cudaError_t launch_batch_k(const DevJob* d_jobs, const uint64_t* d_item_bases, const uint32_t* d_pix_bases,
-                           uint32_t n_jobs, uint32_t max_objects, uint64_t n_items, uint64_t chunk_items,
-                           bool linear, WaveState* wave, DevCounters* d_cnt, cudaStream_t st, WaveLaunch* run);
+cudaError_t launch_batch_k(const JobTable& jobs, uint64_t n_items, uint64_t chunk_items, bool linear,
+                           WaveState* wave, DevCounters* d_cnt, cudaStream_t st, WaveLaunch* run);
 
 // Renders with the wavefront kernels when wave != nullptr, else with the
 // one-thread-per-pixel megakernel.  d_cnt points at 3 counter records:

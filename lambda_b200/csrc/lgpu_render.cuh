@@ -85,11 +85,10 @@ __global__ void __launch_bounds__(128) render_kernel(DevScene S, RenderArgs a, f
 }
 
 // Blocks per SM each wavefront kernel can keep resident (computed once per
-// instantiation; the shading kernel per block size).
+// instantiation).
 struct WaveOccupancy {
   uint32_t sms = 0;
   uint32_t trace, shadow, ptrace, pshadow, gen, fin, fb;
-  uint32_t shade[kMaxShadeBlock / 32 + 1];  // 32, 64, ... threads per block (index block / 32)
 };
 constexpr size_t kTraceSmem = size_t(kSmemStack) * 128 * sizeof(StackEntry);
 
@@ -118,8 +117,6 @@ const WaveOccupancy& wave_occupancy() {
     o.gen = blocks_per_sm(wf_generate_stream<K, J>, 256, 0);
     o.fin = blocks_per_sm(wf_finish<K, J>, 256, 0);
     o.fb = blocks_per_sm(wf_trace_fallback<J>, 128, 0);
-    for (uint32_t b = 1; b <= kMaxShadeBlock / 32; b++)
-      o.shade[b] = blocks_per_sm(wf_shade<K, J, LGPU_MAT_LAMBERTIAN>, 32 * b, 0);
     int dev = 0, sms = 0;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
@@ -131,7 +128,7 @@ const WaveOccupancy& wave_occupancy() {
 // Grids of one render: every SM filled to the kernel's occupancy limit, or
 // to the configured cap for the persistent trace kernels.
 struct WaveGrids {
-  uint32_t trace, shade, shade_block, shadow, gen, ptrace, pshadow, fb, fin;
+  uint32_t trace, shade_block, shadow, gen, ptrace, pshadow, fb, fin;
 };
 
 template <int K, class J>
@@ -144,7 +141,6 @@ WaveGrids wave_grids(const WaveConfig& cfg) {
   WaveGrids g;
   g.trace = o.sms * o.trace;
   g.shade_block = sb;
-  g.shade = o.sms * o.shade[sb / 32];
   g.shadow = o.sms * o.shadow;
   g.gen = o.sms * o.gen;
   g.ptrace = o.sms * cap(o.ptrace);
@@ -194,17 +190,37 @@ inline bool chunk_done(const WaveState& w, uint32_t total) {
 }
 
 constexpr int kItersPerCheck = 4;
+// A chunk whose items all start in the first iteration and whose paths end
+// within this many is launched whole, without asking the device in between
+// (at most WaveLaunch::kSlots, the events of one check).
+constexpr uint32_t kMaxWhole = 16;
+static_assert(kMaxWhole <= WaveLaunch::kSlots && kMaxWhole % 2 == 0, "iterations between two checks");
 
-// Runs iterations of a chunk (issue(w) enqueues one iteration's kernels)
-// until the chunk is done, reading the counters back every kItersPerCheck
-// iterations.  With a graph cache and no per-kernel timing, the
-// kItersPerCheck iterations and the counter readback are captured once as a
-// CUDA graph and replayed; the graph's kernel arguments alternate the two
-// queues, so the state is back in its starting parity after each replay.
+// Runs iterations of a chunk (issue(w, generate) enqueues one iteration's
+// kernels; without `generate` no new paths are due) until the chunk is done.
+//
+// A path takes at most max_scatter + 2 iterations.  If all items fit the
+// queue and that is at most kMaxWhole, all iterations are enqueued at once.
+// Otherwise the counters are read back every kItersPerCheck iterations; with
+// a graph cache and no per-kernel timing, those after the first are captured
+// as a CUDA graph while the device runs the first ones (a capture costs the
+// host as much as the launches it records, 100 us, which a small render does
+// not get back: a 64x64 thumbnail 627 -> 577 us without it), and replayed;
+// the graph's kernel arguments alternate the two queues, so the state is back
+// in its starting parity after each replay.
 template <class Issue>
-cudaError_t run_iterations(WaveState& w, uint32_t total, cudaStream_t st, WaveLaunch* run, Issue issue) {
+cudaError_t run_iterations(WaveState& w, uint32_t total, uint32_t max_scatter, cudaStream_t st, WaveLaunch* run,
+                           Issue issue) {
   size_t const ctl_bytes = kCtlWords * sizeof(uint32_t);
-  bool graph = run->graph && run->cfg.graphs && !run->on;
+  bool const one_fill = total <= w.cap;
+  bool const whole = one_fill && max_scatter + 2ull <= kMaxWhole;
+  int const first = whole ? int((max_scatter + 3u) & ~1u) : kItersPerCheck;
+  for (int k = 0; k < first; k++) {
+    issue(w, k == 0 || !one_fill);
+    swap_queues(w);
+  }
+  cudaMemcpyAsync(w.h_ctl, w.ctl, ctl_bytes, cudaMemcpyDeviceToHost, st);
+  bool graph = !whole && run->graph && run->cfg.graphs && !run->on;
   unsigned long long per_graph = 0;  // kernel launches in one replay
   if (graph) {
     cudaGraph_t gph = nullptr;
@@ -213,7 +229,7 @@ cudaError_t run_iterations(WaveState& w, uint32_t total, cudaStream_t st, WaveLa
     if (e == cudaSuccess) {
       WaveState wc = w;
       for (int k = 0; k < kItersPerCheck; k++) {
-        issue(wc);
+        issue(wc, !one_fill);
         swap_queues(wc);
       }
       cudaMemcpyAsync(w.h_ctl, w.ctl, ctl_bytes, cudaMemcpyDeviceToHost, st);
@@ -239,22 +255,22 @@ cudaError_t run_iterations(WaveState& w, uint32_t total, cudaStream_t st, WaveLa
     }
   }
   for (;;) {
+    cudaError_t e = cudaStreamSynchronize(st);
+    if (e != cudaSuccess) return e;
+    run->harvest();
+    if (chunk_done(w, total)) return cudaSuccess;
     if (graph) {
-      cudaError_t const e = cudaGraphLaunch(run->graph->exec, st);
+      e = cudaGraphLaunch(run->graph->exec, st);
       if (e != cudaSuccess) return e;
       run->graph_launches++;
       run->total += per_graph;
     } else {
       for (int k = 0; k < kItersPerCheck; k++) {
-        issue(w);
+        issue(w, !one_fill);
         swap_queues(w);
       }
       cudaMemcpyAsync(w.h_ctl, w.ctl, ctl_bytes, cudaMemcpyDeviceToHost, st);
     }
-    cudaError_t const e = cudaStreamSynchronize(st);
-    if (e != cudaSuccess) return e;
-    run->harvest();
-    if (chunk_done(w, total)) return cudaSuccess;
   }
 }
 
@@ -263,7 +279,7 @@ cudaError_t run_iterations(WaveState& w, uint32_t total, cudaStream_t st, WaveLa
 // new paths behind the queue up to its capacity (plan + generate), then
 // advances every queued path by one segment (trace, shade, shadow); the
 // chunk's (sample, pixel) results are then added to the film.
-template <int K, class J>
+template <int K, bool REC, class J>
 cudaError_t wave_chunk(const J& jobs, WaveState& w, uint64_t c0, uint32_t total, bool linear,
                        DevCounters* d_cnt, cudaStream_t st, WaveLaunch* run) {
   DevCounters* const c_closest = run->on ? d_cnt + 1 : d_cnt;
@@ -272,10 +288,10 @@ cudaError_t wave_chunk(const J& jobs, WaveState& w, uint64_t c0, uint32_t total,
   w.c0 = c0;
   wf_stream_init<<<1, 32, 0, st>>>(w);
   run->total++;
-  cudaError_t e = run_iterations(w, total, st, run, [&](const WaveState& wi) {
+  cudaError_t e = run_iterations(w, total, jobs.max_scatter(), st, run, [&](const WaveState& wi, bool generate) {
     wf_finish<K, J><<<g.fin, 256, 0, st>>>(jobs, wi, d_cnt);
     wf_plan<<<1, 1, 0, st>>>(wi, total);
-    wf_generate_stream<K, J><<<g.gen, 256, 0, st>>>(jobs, wi, d_cnt);
+    if (generate) wf_generate_stream<K, J><<<g.gen, 256, 0, st>>>(jobs, wi, d_cnt);
     run->begin(0, st);
     launch_closest<K>(jobs, wi, g, linear, c_closest, st);
     run->end(0, st);
@@ -283,20 +299,22 @@ cudaError_t wave_chunk(const J& jobs, WaveState& w, uint64_t c0, uint32_t total,
     // one block per queue chunk, not persistent: a block's warps finish
     // their material-sorted groups at different times, and a persistent
     // block would hold the fast ones at the next chunk's sort barrier.
-    // Three launches, each with one material type's code (the rest, Blinn,
-    // thin film), so an SM's warps share their instructions; the first
-    // lists the Blinn and thin-film hits for the other two.
+    // Up to three launches, each with one material type's code (the rest,
+    // Blinn, thin film; the last two only if a scene has such a material), so
+    // an SM's warps share their instructions; the first lists the Blinn and
+    // thin-film hits for the other two.
     uint32_t const sg = (wi.cap + g.shade_block - 1) / g.shade_block;
-    wf_shade<K, J, LGPU_MAT_LAMBERTIAN><<<sg, g.shade_block, 0, st>>>(jobs, wi, d_cnt);
-    wf_shade<K, J, LGPU_MAT_BLINN><<<sg, g.shade_block, 0, st>>>(jobs, wi, d_cnt);
-    wf_shade<K, J, LGPU_MAT_THINFILM><<<sg, g.shade_block, 0, st>>>(jobs, wi, d_cnt);
+    bool const blinn = jobs.has_material(LGPU_MAT_BLINN), film = jobs.has_material(LGPU_MAT_THINFILM);
+    wf_shade<K, J, LGPU_MAT_LAMBERTIAN, REC><<<sg, g.shade_block, 0, st>>>(jobs, wi, d_cnt);
+    if (blinn) wf_shade<K, J, LGPU_MAT_BLINN, REC><<<sg, g.shade_block, 0, st>>>(jobs, wi, d_cnt);
+    if (film) wf_shade<K, J, LGPU_MAT_THINFILM, REC><<<sg, g.shade_block, 0, st>>>(jobs, wi, d_cnt);
     run->end(2, st);
     run->begin(1, st);
     if (linear) wf_shadow<K, J><<<g.shadow, 128, kTraceSmem, st>>>(jobs, wi, c_shadow);
     else wf_trace_persistent<true, K, J><<<g.pshadow, 128, kTraceSmem, st>>>(jobs, wi, c_shadow);
     run->end(1, st);
-    // finish, plan, generate, shade (3), shadow
-    run->total += 7 + closest_launches(jobs, linear);
+    // finish, plan, shade, shadow
+    run->total += 4 + (generate ? 1 : 0) + (blinn ? 1 : 0) + (film ? 1 : 0) + closest_launches(jobs, linear);
   });
   if (e != cudaSuccess) return e;
   wf_finish<K, J><<<g.fin, 256, 0, st>>>(jobs, w, d_cnt);
@@ -326,7 +344,7 @@ cudaError_t run_wave(const J& jobs, WaveState w, uint64_t n_items, uint64_t chun
   if (e == cudaSuccess && w.film64) e = cudaMemsetAsync(w.film64, 0, sizeof(double) * 3 * size_t(w.npix), st);
   for (uint64_t c0 = 0; c0 < n_items && e == cudaSuccess; c0 += chunk_items) {
     uint32_t const total = uint32_t(n_items - c0 < chunk_items ? n_items - c0 : chunk_items);
-    e = wave_chunk<K>(jobs, w, c0, total, linear, d_cnt, st, run);
+    e = wave_chunk<K, false>(jobs, w, c0, total, linear, d_cnt, st, run);
   }
   if (e == cudaSuccess) e = finalize_film<K>(jobs, w, st, run);
   return e;
@@ -349,10 +367,8 @@ cudaError_t launch_render_k(const DevScene& S, const RenderArgs& a, WaveState* w
 }
 
 template <int K>
-cudaError_t launch_batch_k(const DevJob* d_jobs, const uint64_t* d_item_bases, const uint32_t* d_pix_bases,
-                           uint32_t n_jobs, uint32_t max_objects, uint64_t n_items, uint64_t chunk_items,
-                           bool linear, WaveState* wave, DevCounters* d_cnt, cudaStream_t st, WaveLaunch* run) {
-  JobTable const jobs{d_jobs, d_item_bases, d_pix_bases, n_jobs, max_objects};
+cudaError_t launch_batch_k(const JobTable& jobs, uint64_t n_items, uint64_t chunk_items, bool linear,
+                           WaveState* wave, DevCounters* d_cnt, cudaStream_t st, WaveLaunch* run) {
   return run_wave<K>(jobs, *wave, n_items, chunk_items, linear, d_cnt, st, run);
 }
 

@@ -109,6 +109,7 @@ struct DevScene {
   uint32_t max_stack;  // max over meshes of DevMesh::max_stack
   uint32_t tlas_max_stack;
   uint32_t n_bins, hero_k;
+  uint32_t mat_types;  // bit t set: a material of type t (lgpu_material_type)
   float lambda_inf, lambda_sup, lambda_delta;
   // the correctly rounded reciprocals of lambda_delta and of the hero
   // wavelength's density 1 / (lambda_sup - lambda_inf), or 0 where div_by

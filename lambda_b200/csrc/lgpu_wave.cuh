@@ -362,6 +362,12 @@ __device__ __forceinline__ void shadow_done(const WaveState& w, uint32_t s, bool
 // which each lane popped, sorted and pushed by itself.
 constexpr int kRefill = 12;
 constexpr int kTriLanes = 6, kObjLanes = 6;
+// A launch with fewer rays than lanes is as long as its longest warp, and a
+// warp with fewer rays takes fewer and shorter steps: closest-hit rays are
+// then spread over all warps, 8 to each at least (131,072 rays of the
+// inverse-rendering scene: 185 -> 165 us a launch, 16: 175 us; shadow rays
+// gain 10 % there but the kernel then spills and loses 4 % on full queues).
+constexpr uint32_t kMinShare = 8;
 
 // Occupancy (measured best): 7 blocks of 128 per SM (72 registers) for
 // any-hit queries (6: +11 %, 8: the same), 6 (80 registers) for closest-hit
@@ -385,6 +391,11 @@ __global__ void __launch_bounds__(128, ANY ? 7 : 6) wf_trace_persistent(J jobs, 
   // lanes without work that make the warp stop for new rays; once there are
   // none left, any lane that finishes
   int wait = kRefill;
+  // Fewer closest-hit rays than lanes: each warp takes its share of them, at
+  // least kMinShare, at once.
+  uint32_t const warps = gridDim.x * (blockDim.x >> 5);
+  uint32_t const share = ANY ? 32u : max(kMinShare, min(32u, (n + warps - 1u) / warps));
+  bool const on = uint32_t(lane) < share;
   uint32_t idx = 0, jb = 0;
   auto accept = [&](uint32_t face, float b0, float b1, float b2, f3 pl, float z) {
     if (!ANY) store_hit_point(w, idx, face, b0, b1, b2, pl, z);
@@ -461,7 +472,7 @@ __global__ void __launch_bounds__(128, ANY ? 7 : 6) wf_trace_persistent(J jobs, 
           }
         }
       }
-      unsigned idle = __ballot_sync(FULL, t.kind == kLaneIdle);
+      unsigned idle = __ballot_sync(FULL, t.kind == kLaneIdle && on);
       if (wait == kRefill && idle) {
         uint32_t const want = uint32_t(__popc(idle));
         int const leader = __ffs(idle) - 1;
@@ -470,7 +481,7 @@ __global__ void __launch_bounds__(128, ANY ? 7 : 6) wf_trace_persistent(J jobs, 
         base = __shfl_sync(FULL, base, leader);
         uint32_t const got = min(base < n ? n - base : 0u, want);
         uint32_t const k = uint32_t(__popc(idle & ((1u << lane) - 1u)));
-        if (t.kind == kLaneIdle && k < got) {
+        if (t.kind == kLaneIdle && on && k < got) {
           idx = base + k;
           if (J::kMulti) jb = ANY ? w.s_job[idx] : w.in.job[idx];
           if (ANY) {
@@ -486,9 +497,9 @@ __global__ void __launch_bounds__(128, ANY ? 7 : 6) wf_trace_persistent(J jobs, 
           trace_begin(jobs.scene(jb), t, st);
         }
         rays += got;
-        if (base + want >= n) wait = 0;
-        idle = __ballot_sync(FULL, t.kind == kLaneIdle);
+        if (base + want >= n || share < 32u) wait = 0;
       }
+      idle = __ballot_sync(FULL, t.kind == kLaneIdle);
       if (wait != kRefill) {
         if (idle == FULL) break;
         wait = __popc(idle) + 1;
@@ -632,7 +643,8 @@ __device__ __forceinline__ void list_material_groups(const WaveState& w, uint32_
 // paths that hit that material (its code alone, the others' branches fold
 // away); MT = LGPU_MAT_LAMBERTIAN: every other path (misses, emitters,
 // Lambertian and unshaded materials).  The three specialised launches
-// together shade every path once.
+// together shade every path once.  REC: the primal pass of an adjoint, which
+// records what the replay reads.
 template <int MT>
 __device__ __forceinline__ bool shade_group(uint32_t group) {
   if (MT < 0) return true;
@@ -651,7 +663,7 @@ __device__ __forceinline__ bool shade_group(uint32_t group) {
 // frame's first launch but 7 % slower on the box room's; 6 and 5 before.
 // Benchmark frame: first launch 48.2 -> 39.2 ms, Blinn list 16.5 -> 14.9,
 // thin-film list 16.3 -> 14.3; box room 605 -> 472 us.
-template <int K, class J, int MT = -1>
+template <int K, class J, int MT, bool REC>
 __global__ void __launch_bounds__(kMaxShadeBlock, 4) wf_shade(J jobs, WaveState w, DevCounters* cnt) {
   uint32_t const n = *w.n_in;
   uint32_t const cap = w.cap;
@@ -715,7 +727,7 @@ __global__ void __launch_bounds__(kMaxShadeBlock, 4) wf_shade(J jobs, WaveState 
       prev_s = rc.w;
       uint32_t const obj = w.hobj[i];
       size_t const v_at = size_t(depth) * w.v_items + item;
-      if (w.v_obj) w.v_obj[v_at] = UINT32_MAX;
+      if (REC && w.v_obj) w.v_obj[v_at] = UINT32_MAX;
       if (obj != UINT32_MAX) {
         HitRec const h = load_hit(w.hita, w.hitb, i, obj);
         Ray const r = make_ray(in.ra[i], rb);
@@ -734,7 +746,7 @@ __global__ void __launch_bounds__(kMaxShadeBlock, 4) wf_shade(J jobs, WaveState 
           }
         } else if (depth <= a.max_scatter) {
           kind = kScatter;
-          if (w.v_obj) {
+          if (REC && w.v_obj) {
             w.v_obj[v_at] = obj;
             w.v_hita[v_at] = make_float4(__uint_as_float(h.face), h.b0, h.b1, h.b2);
             w.v_hitb[v_at] = make_float4(h.pl.x, h.pl.y, h.pl.z, h.z);
@@ -799,7 +811,7 @@ __global__ void __launch_bounds__(kMaxShadeBlock, 4) wf_shade(J jobs, WaveState 
     }
     if (shadow) {
       if (J::kMulti) w.s_job[s_pos] = jb;
-      if (w.vis) {
+      if (REC) {
         w.s_item[s_pos] = item;
         w.s_depth[s_pos] = depth;
       }
