@@ -435,8 +435,11 @@ cudaError_t replay_chunk(const OneJob& jobs, WaveState& w, uint64_t c0, uint32_t
     uint32_t const sg = (wi.cap + gr.shade_block - 1) / gr.shade_block;
     wf_shade_adjoint<K, LGPU_MAT_LAMBERTIAN><<<sg, gr.shade_block, 0, st>>>(jobs, wi, g);
     bool const blinn = jobs.has_material(LGPU_MAT_BLINN), film = jobs.has_material(LGPU_MAT_THINFILM);
+    cudaStream_t const fs = blinn && film ? run->fork_side(st) : st;
+    if (film) wf_shade_adjoint<K, LGPU_MAT_THINFILM><<<sg, gr.shade_block, 0, fs>>>(jobs, wi, g);
+    if (fs != st) run->end_side();
     if (blinn) wf_shade_adjoint<K, LGPU_MAT_BLINN><<<sg, gr.shade_block, 0, st>>>(jobs, wi, g);
-    if (film) wf_shade_adjoint<K, LGPU_MAT_THINFILM><<<sg, gr.shade_block, 0, st>>>(jobs, wi, g);
+    run->wait_side(st);
     run->end(2, st);
     // plan, shade
     run->total += 2 + (generate ? 1 : 0) + (blinn ? 1 : 0) + (film ? 1 : 0);

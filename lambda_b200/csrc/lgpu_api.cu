@@ -116,6 +116,8 @@ struct lgpu_ctx {
   WaveConfig cfg;     // launch shape of the wavefront
   GraphCache graph;   // captured bounce stages
   cudaEvent_t ev_fork = nullptr, ev_join = nullptr;
+  cudaStream_t beside = nullptr;  // the wavefront's shadow and film launches
+  cudaEvent_t ev_bfork = nullptr, ev_bjoin = nullptr;
   cudaStream_t side = nullptr;  // batches: the megakernel jobs
   bool keep_counters = false;   // the counters were reset by the caller of a nested render
 
@@ -341,6 +343,9 @@ int prepare_launch(lgpu_ctx* ctx, bool timing) {
   ctx->launch.reset(timing);
   ctx->launch.cfg = ctx->cfg;
   ctx->launch.graph = &ctx->graph;
+  ctx->launch.side = ctx->beside;
+  ctx->launch.fork = ctx->ev_bfork;
+  ctx->launch.join = ctx->ev_bjoin;
   return LGPU_OK;
 }
 
@@ -896,6 +901,9 @@ int lgpu_create(int device, lgpu_ctx** out) {
   if (e == cudaSuccess) e = cudaEventCreate(&ctx->ev1);
   if (e == cudaSuccess) e = cudaEventCreateWithFlags(&ctx->ev_fork, cudaEventDisableTiming);
   if (e == cudaSuccess) e = cudaEventCreateWithFlags(&ctx->ev_join, cudaEventDisableTiming);
+  if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&ctx->beside, cudaStreamNonBlocking);
+  if (e == cudaSuccess) e = cudaEventCreateWithFlags(&ctx->ev_bfork, cudaEventDisableTiming);
+  if (e == cudaSuccess) e = cudaEventCreateWithFlags(&ctx->ev_bjoin, cudaEventDisableTiming);
   if (e == cudaSuccess) e = cudaMalloc(&ctx->counters, 3 * sizeof(DevCounters));
   if (e == cudaSuccess) e = cudaMallocHost(&ctx->h_ctl, kCtlWords * sizeof(uint32_t));
   if (e != cudaSuccess) {
@@ -938,6 +946,12 @@ void lgpu_destroy(lgpu_ctx* ctx) {
   if (ctx->ev1) cudaEventDestroy(ctx->ev1);
   if (ctx->ev_fork) cudaEventDestroy(ctx->ev_fork);
   if (ctx->ev_join) cudaEventDestroy(ctx->ev_join);
+  if (ctx->beside) {
+    cudaStreamSynchronize(ctx->beside);
+    cudaStreamDestroy(ctx->beside);
+  }
+  if (ctx->ev_bfork) cudaEventDestroy(ctx->ev_bfork);
+  if (ctx->ev_bjoin) cudaEventDestroy(ctx->ev_bjoin);
   ctx->graph.release();
   for (auto& k : ctx->launch.ev)
     for (auto& s : k)

@@ -60,7 +60,8 @@ struct Ray {
   f3 p, u, inv;
 };
 __device__ __forceinline__ float inv_or_max(float u) {
-  return u != 0.f ? dv(1.f, u) : kFltMax;
+  float const r = __frcp_rn(u);  // 1 / u, correctly rounded as the division
+  return u != 0.f ? r : kFltMax;
 }
 __device__ __forceinline__ Ray make_ray(f3 p, f3 u) {
   return Ray{p, u, f3{inv_or_max(u.x), inv_or_max(u.y), inv_or_max(u.z)}};

@@ -36,19 +36,22 @@ struct PathBuf {
   float4* gw;       // K/4 words, path replay: dL/d(radiance) per hero wavelength
 };
 
-// Counters of the wavefront renderer (WaveState::ctl).
+// Counters of the wavefront renderer (WaveState::ctl).  The pairs alternate
+// between iterations (WaveState::par): an iteration's shadow rays and ended
+// paths are worked on beside the next one's closest-hit launch.
 constexpr int kCtlCountA = 0;    // queue lengths of the two PathBufs
 constexpr int kCtlCountB = 1;
-constexpr int kCtlShadow = 2;    // shadow rays
-constexpr int kCtlFetch = 3;     // 2 work counters of the persistent trace kernels
-constexpr int kCtlFallback = 5;  // rays re-traced in the reference's object order
-constexpr int kCtlEnded = 6;     // ended paths
-constexpr int kCtlNext = 7;      // next work item to start
-constexpr int kCtlNew = 8;       // plan of the next generate: new paths,
-constexpr int kCtlFirst = 9;     //   their first work item,
-constexpr int kCtlPos = 10;      //   their first queue position
-constexpr int kCtlListB = 11;    // queue entries that hit a Blinn material
-constexpr int kCtlListT = 12;    //   and a thin-film one (shading lists)
+constexpr int kCtlShadow = 2;    // pair: shadow rays
+constexpr int kCtlFetch = 4;     // work counter of the closest-hit kernel,
+constexpr int kCtlSFetch = 5;    // pair: of the shadow kernel
+constexpr int kCtlFallback = 7;  // rays re-traced in the reference's object order
+constexpr int kCtlEnded = 8;     // pair: ended paths
+constexpr int kCtlNext = 10;     // next work item to start
+constexpr int kCtlNew = 11;      // plan of the next generate: new paths,
+constexpr int kCtlFirst = 12;    //   their first work item,
+constexpr int kCtlPos = 13;      //   their first queue position
+constexpr int kCtlListB = 14;    // queue entries that hit a Blinn material
+constexpr int kCtlListT = 15;    //   and a thin-film one (shading lists)
 constexpr int kCtlWords = 16;
 constexpr uint32_t kNoShadow = 0xFFFFFFFFu;
 
@@ -58,6 +61,7 @@ struct WaveState {
   uint32_t npix;       // pixels of the frame (of all frames of a batch)
   uint32_t n_samples;  // samples per pixel in one chunk of the frame
   uint64_t c0;         // first work item of the current chunk
+  uint32_t par;        // which counter of each pair this iteration uses
   PathBuf in, out;     // current and next queue, swapped every iteration
   uint32_t* n_in;      // queue lengths (in ctl), swapped with the queues
   uint32_t* n_out;
@@ -147,6 +151,10 @@ struct WaveLaunch {
   static constexpr int kSlots = 16;
   WaveConfig cfg;
   GraphCache* graph = nullptr;
+  // the stream of the shadow and film launches and its fork and join events
+  cudaStream_t side = nullptr;
+  cudaEvent_t fork = nullptr, join = nullptr;
+  bool forked = false;  // side work that st does not wait for yet
   unsigned long long graph_launches = 0;
   bool on = false;
   unsigned long long total = 0;  // kernel launches
@@ -156,6 +164,7 @@ struct WaveLaunch {
   unsigned long long launches[3] = {0, 0, 0};
   void reset(bool timing) {
     on = timing;
+    forked = false;
     total = 0;
     graph_launches = 0;
     for (int k = 0; k < 3; k++) {
@@ -163,6 +172,24 @@ struct WaveLaunch {
       ms[k] = 0.0;
       launches[k] = 0;
     }
+  }
+  // The side stream, ordered after what was enqueued on st; st itself with
+  // per-kernel timing (the kernels are then timed one by one).
+  cudaStream_t fork_side(cudaStream_t st) {
+    if (on || !side) return st;
+    cudaEventRecord(fork, st);
+    cudaStreamWaitEvent(side, fork, 0);
+    forked = true;
+    return side;
+  }
+  // after the side stream's launches
+  void end_side() {
+    if (!on && side) cudaEventRecord(join, side);
+  }
+  // st waits for them, if it does not yet
+  void wait_side(cudaStream_t st) {
+    if (forked) cudaStreamWaitEvent(st, join, 0);
+    forked = false;
   }
   void begin(int k, cudaStream_t st) {
     if (on) cudaEventRecord(ev[k][used[k]][0], st);

@@ -4,9 +4,6 @@
 // its state at index i of the `in` buffers (field-major, so a warp's access
 // to one field is one coalesced transaction).  Each iteration
 //
-//   wf_finish<K>          ended paths of the last iteration (with the light
-//                         sample of their last vertex if its shadow ray got
-//                         through) -> XYZ of their (sample, pixel) film entry
 //   wf_plan               how many new paths fit behind the queue
 //   wf_generate_stream<K> camera ray + hero wavelengths of the new paths,
 //                         appended to the queue
@@ -19,7 +16,12 @@
 //   wf_shadow / wf_trace_persistent<true>
 //                         any-hit test of the shadow rays: one visibility
 //                         byte per ray
+//   wf_finish<K>          ended paths (with the light sample of their last
+//                         vertex if its shadow ray got through) -> XYZ of
+//                         their (sample, pixel) film entry
 //
+// the last two on a second stream, beside the next iteration's plan, new
+// paths and closest hits (its shading waits for them);
 // then the host swaps `in` and `out`.  No path keeps a fixed slot, so no
 // access is scattered.  Each path draws its random numbers from its own
 // counter-based stream in the order of Renderer::tracePath
@@ -99,14 +101,13 @@ __global__ void wf_stream_init(WaveState w) {
   if (blockIdx.x == 0 && threadIdx.x == 0) {
     *w.n_in = 0;
     *w.n_out = 0;
-    w.ctl[kCtlEnded] = 0;
     w.ctl[kCtlNext] = 0;
   }
 }
 
-// Runs after wf_finish: plans the next generate (as many new paths as fit
-// behind the queue, up to the remaining work items) and clears the
-// per-iteration counters.
+// Plans the next generate (as many new paths as fit behind the queue, up to
+// the remaining work items) and clears the iteration's counters.  The other
+// counters of the pairs may still be in use by the last iteration.
 __global__ void wf_plan(WaveState w, uint32_t total) {
   uint32_t const n_in = *w.n_in, next = w.ctl[kCtlNext];
   uint32_t const room = w.cap - n_in;
@@ -118,11 +119,11 @@ __global__ void wf_plan(WaveState w, uint32_t total) {
   w.ctl[kCtlNext] = next + n_new;
   *w.n_in = n_in + n_new;
   *w.n_out = 0;
-  w.ctl[kCtlShadow] = 0;
+  w.ctl[kCtlShadow + w.par] = 0;
   w.ctl[kCtlFetch] = 0;
-  w.ctl[kCtlFetch + 1] = 0;
+  w.ctl[kCtlSFetch + w.par] = 0;
   w.ctl[kCtlFallback] = 0;
-  w.ctl[kCtlEnded] = 0;
+  w.ctl[kCtlEnded + w.par] = 0;
   w.ctl[kCtlListB] = 0;
   w.ctl[kCtlListT] = 0;
 }
@@ -192,7 +193,7 @@ __global__ void __launch_bounds__(256) wf_generate_stream(J jobs, WaveState w, D
 // div_by.  Benchmark frame: 16.0 -> 11.2 ms.
 template <int K, class J>
 __global__ void __launch_bounds__(256) wf_finish(J jobs, WaveState w, DevCounters* cnt) {
-  uint32_t const n = w.ctl[kCtlEnded];
+  uint32_t const n = w.ctl[kCtlEnded + w.par];
   uint32_t const cap = w.cap;
   uint32_t nonfinite = 0;
   for (uint32_t e = blockIdx.x * blockDim.x + threadIdx.x; e < n; e += gridDim.x * blockDim.x) {
@@ -210,7 +211,7 @@ __global__ void __launch_bounds__(256) wf_finish(J jobs, WaveState w, DevCounter
 #pragma unroll 1
     for (int q = 0; q < K / 4; q++) {
       float4 const a4 = w.e_acc[q * cap + e];
-      float4 const p4 = lit ? w.s_prev[q * cap + sx_i] : make_float4(0.f, 0.f, 0.f, 0.f);
+      float4 const p4 = lit ? w.s_contrib[q * cap + sx_i] : make_float4(0.f, 0.f, 0.f, 0.f);
       float acc[4] = {a4.x, a4.y, a4.z, a4.w};
       float const pend[4] = {p4.x, p4.y, p4.z, p4.w};
 #pragma unroll
@@ -381,8 +382,8 @@ __global__ void __launch_bounds__(128, ANY ? 7 : 6) wf_trace_persistent(J jobs, 
   st.ws = wsave + threadIdx.x;
   uint32_t rays = 0, nodes = 0;  // of the warp
   uint32_t tris = 0, insts = 0;
-  uint32_t const n = ANY ? w.ctl[kCtlShadow] : *w.n_in;
-  uint32_t* fetch = w.ctl + kCtlFetch + (ANY ? 1 : 0);
+  uint32_t const n = ANY ? w.ctl[kCtlShadow + w.par] : *w.n_in;
+  uint32_t* fetch = w.ctl + (ANY ? kCtlSFetch + w.par : uint32_t(kCtlFetch));
   uint32_t const cap = w.cap;
   unsigned const FULL = 0xFFFFFFFFu;
   int const lane = threadIdx.x & 31;
@@ -795,8 +796,8 @@ __global__ void __launch_bounds__(kMaxShadeBlock, 4) wf_shade(J jobs, WaveState 
     // compacted appends: next queue, ended list, shadow queue
     bool const ended = live && !cont;
     uint32_t const o_pos = warp_append(w.n_out, cont);
-    uint32_t const e_pos = warp_append(w.ctl + kCtlEnded, ended);
-    uint32_t const s_pos = warp_append(w.ctl + kCtlShadow, shadow);
+    uint32_t const e_pos = warp_append(w.ctl + kCtlEnded + w.par, ended);
+    uint32_t const s_pos = warp_append(w.ctl + kCtlShadow + w.par, shadow);
     if (!live) continue;
     // the path's records first: the wavelength loop below then has only the
     // scalars of its spectra to keep in registers
@@ -894,7 +895,7 @@ __global__ void __launch_bounds__(128) wf_shadow(J jobs, WaveState w, DevCounter
   SplitStack st{smem_stack + threadIdx.x, blockDim.x, lm, 0, 0u};
   TravStats ts{0u, 0u, 0u, 0u};
   uint32_t rays = 0;
-  uint32_t const n = w.ctl[kCtlShadow];
+  uint32_t const n = w.ctl[kCtlShadow + w.par];
   uint32_t const cap = w.cap;
   for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
     uint32_t const jb = J::kMulti ? w.s_job[i] : 0u;
