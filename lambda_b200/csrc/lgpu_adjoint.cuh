@@ -186,16 +186,15 @@ __global__ void __launch_bounds__(256) wf_replay_generate(OneJob jobs, WaveState
 }
 
 // One vertex of the replay: the same random decisions as wf_shade, the
-// visibility recorded by the primal pass, gradients accumulated.  Three
-// launches by material like wf_shade's (MT: Lambertian and the rest, which
-// also lists the others; Blinn; thin film).
+// visibility recorded by the primal pass, gradients accumulated.  The
+// launches by material are wf_shade's (MT); kShadeRest only fills the lists.
 //
 // Bound by issue and by instruction fetch (5 of 16 stalls in one launch for
 // all materials, with the gradient code of each in every block).  64x64
 // thin-film tiles under 64 spheres, 512x512, 32 spp: one launch with
 // forward-mode dual numbers 18.8 ms, closed-form thin-film derivatives 10.7
-// ms, three launches 6.6 ms (4 blocks of 256 per SM; 3
-// and 5: +5 %); the bins' atomics are no bound (without
+// ms, launches by material 6.6 ms (4 blocks of 256 per SM; 3 and 5: +5 %),
+// Lambertian hits in a list 6.4 ms; the bins' atomics are no bound (without
 // them 18.4 of the 18.8 ms).
 template <int K, int MT>
 __global__ void __launch_bounds__(kMaxShadeBlock, 4) wf_shade_adjoint(OneJob jobs, WaveState w, AdjointArgs g) {
@@ -207,26 +206,24 @@ __global__ void __launch_bounds__(kMaxShadeBlock, 4) wf_shade_adjoint(OneJob job
   PathBuf const& out = w.out;
   float const omega = S.lambda_sup - S.lambda_inf;
   float const step = omega / float(K);
-  constexpr bool kList = MT == LGPU_MAT_BLINN || MT == LGPU_MAT_THINFILM;
-  uint32_t const n_loop = kList ? w.ctl[MT == LGPU_MAT_BLINN ? kCtlListB : kCtlListT] : n;
+  constexpr bool kList = kShadeLists<MT>;
+  uint32_t const n_loop = kList ? shade_list_length<MT>(w) : n;
   for (uint32_t base = blockIdx.x * blockDim.x; base < n_loop; base += gridDim.x * blockDim.x) {
-    uint32_t group = 1u + MT, i;
+    uint32_t group = 0, i;
     if (kList) {
-      uint32_t const j = base + threadIdx.x;
-      i = j < n_loop ? w.shade_list[MT == LGPU_MAT_BLINN ? j : cap - 1u - j] : UINT32_MAX;
+      i = shade_list_entry<MT>(w, base + threadIdx.x, n_loop);
     } else {
       i = material_order(jobs, w, base, n, &group, [&](uint32_t q) {
         return w.v_obj ? w.v_obj[size_t(__float_as_uint(in.rb[q].w)) * w.v_items + in.rc[q].z] : w.hobj[q];
       });
-      list_material_groups(w, i, group);
+      if (MT == kShadeRest) {
+        // misses and emitters end their paths without a gradient
+        list_material_groups(w, i, group);
+        continue;
+      }
     }
-    bool const live = i < n && shade_group<MT>(group);
-    auto material = [&](uint32_t idx) {
-      DevMaterial x = S.mats[idx];
-      if (kList) x.type = MT;
-      if (!kList && (x.type == LGPU_MAT_BLINN || x.type == LGPU_MAT_THINFILM)) x.type = LGPU_MAT_MICROFACET;
-      return x;
-    };
+    bool const live = i < n;
+    auto material = [&](uint32_t idx) { return shade_material<MT>(S, idx); };
     bool cont = false, scatter = false, visible = false;
     f3 np = f3{0.f, 0.f, 0.f}, nd = f3{0.f, 0.f, 1.f};
     float lis_scale = 0.f, m_scale = 0.f, hero = 0.f;
@@ -304,16 +301,7 @@ __global__ void __launch_bounds__(kMaxShadeBlock, 4) wf_shade_adjoint(OneJob job
         }
       }
     }
-    // what this launch's materials leave of the BSDF cases and lobes
-    if (MT == LGPU_MAT_LAMBERTIAN) {
-      bl.kind = bl.kind ? 1 : 0;
-      ms.lobe = ms.lobe ? 1 : 0;
-    } else if (MT == LGPU_MAT_BLINN) {
-      bl.kind = bl.kind == 2 ? 2 : 3;
-    } else {
-      bl.kind = bl.kind ? 4 : 0;
-      ms.lobe = ms.lobe ? 4 : 0;
-    }
+    shade_cases<MT>(bl, ms);
     uint32_t const o_pos = warp_append(w.n_out, cont);
     if (!scatter) continue;
     if (cont) {
@@ -433,16 +421,22 @@ cudaError_t replay_chunk(const OneJob& jobs, WaveState& w, uint64_t c0, uint32_t
     run->begin(2, st);
     // one block per queue chunk (see wave_chunk)
     uint32_t const sg = (wi.cap + gr.shade_block - 1) / gr.shade_block;
-    wf_shade_adjoint<K, LGPU_MAT_LAMBERTIAN><<<sg, gr.shade_block, 0, st>>>(jobs, wi, g);
     bool const blinn = jobs.has_material(LGPU_MAT_BLINN), film = jobs.has_material(LGPU_MAT_THINFILM);
-    cudaStream_t const fs = blinn && film ? run->fork_side(st) : st;
-    if (film) wf_shade_adjoint<K, LGPU_MAT_THINFILM><<<sg, gr.shade_block, 0, fs>>>(jobs, wi, g);
-    if (fs != st) run->end_side();
-    if (blinn) wf_shade_adjoint<K, LGPU_MAT_BLINN><<<sg, gr.shade_block, 0, st>>>(jobs, wi, g);
+    bool const lists = blinn || film;
+    if (!lists) {
+      wf_shade_adjoint<K, LGPU_MAT_LAMBERTIAN><<<sg, gr.shade_block, 0, st>>>(jobs, wi, g);
+    } else {
+      wf_shade_adjoint<K, kShadeRest><<<sg, gr.shade_block, 0, st>>>(jobs, wi, g);
+      cudaStream_t const fs = run->fork_side(st);
+      if (film) wf_shade_adjoint<K, LGPU_MAT_THINFILM><<<sg, gr.shade_block, 0, fs>>>(jobs, wi, g);
+      if (blinn) wf_shade_adjoint<K, LGPU_MAT_BLINN><<<sg, gr.shade_block, 0, film ? st : fs>>>(jobs, wi, g);
+      run->end_side();
+      wf_shade_adjoint<K, kShadeLamb><<<sg, gr.shade_block, 0, st>>>(jobs, wi, g);
+    }
     run->wait_side(st);
     run->end(2, st);
     // plan, shade
-    run->total += 2 + (generate ? 1 : 0) + (blinn ? 1 : 0) + (film ? 1 : 0);
+    run->total += 2 + (generate ? 1 : 0) + (lists ? 1 : 0) + (blinn ? 1 : 0) + (film ? 1 : 0);
   });
 }
 

@@ -277,6 +277,7 @@ size_t wave_layout(uint8_t* base, uint32_t cap, uint32_t K, uint32_t npix, uint6
   ws.s_job = batch ? c.take<uint32_t>(n) : nullptr;
   ws.fb_queue = c.take<uint32_t>(n);
   ws.shade_list = c.take<uint32_t>(n);
+  ws.shade_list2 = c.take<uint32_t>(n);
   ws.ctl = c.take<uint32_t>(kCtlWords);
   ws.film = c.take<float>(3 * size_t(npix));
   ws.film64 = fp64 ? c.take<double>(3 * size_t(npix)) : nullptr;
@@ -612,7 +613,7 @@ bool timing_requested(const lgpu_render_params* p) {
 // The material types a scene has, one bit each.
 uint32_t material_types(const std::vector<DevMaterial>& mats) {
   uint32_t t = 0;
-  for (const DevMaterial& m : mats) t |= 1u << m.type;
+  for (const DevMaterial& m : mats) t |= 1u << (uint32_t(m.type) & 31u);
   return t;
 }
 

@@ -51,8 +51,9 @@ constexpr int kCtlNew = 11;      // plan of the next generate: new paths,
 constexpr int kCtlFirst = 12;    //   their first work item,
 constexpr int kCtlPos = 13;      //   their first queue position
 constexpr int kCtlListB = 14;    // queue entries that hit a Blinn material
-constexpr int kCtlListT = 15;    //   and a thin-film one (shading lists)
-constexpr int kCtlWords = 16;
+constexpr int kCtlListT = 15;    //   a thin-film one,
+constexpr int kCtlListL = 16;    //   any other scattering one (shading lists)
+constexpr int kCtlWords = 24;
 constexpr uint32_t kNoShadow = 0xFFFFFFFFu;
 
 // Device buffers of the wavefront renderer; the context owns them.
@@ -80,6 +81,7 @@ struct WaveState {
   uint32_t* fb_queue;  // cap: `in` indices re-traced in the reference's object order
   uint32_t* shade_list;  // cap: `in` positions of the Blinn hits (from the front) and
                          // of the thin-film hits (from the back), for their shading launches
+  uint32_t* shade_list2; // cap: of the Lambertian and unshaded hits
   uint32_t* ctl;       // kCtlWords counters
   uint32_t* h_ctl;     // pinned host copy of ctl
   float* sbuf;         // 3 per work item of a chunk: XYZ of every (sample, pixel)

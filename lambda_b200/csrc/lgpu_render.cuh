@@ -303,18 +303,20 @@ cudaError_t wave_chunk(const J& jobs, WaveState& w, uint64_t c0, uint32_t total,
     // one block per queue chunk, not persistent: a block's warps finish
     // their material-sorted groups at different times, and a persistent
     // block would hold the fast ones at the next chunk's sort barrier.
-    // Up to three launches, each with one material type's code (the rest,
-    // Blinn, thin film; the last two only if a scene has such a material), so
-    // an SM's warps share their instructions; the first lists the Blinn and
-    // thin-film hits for the other two.
     uint32_t const sg = (wi.cap + g.shade_block - 1) / g.shade_block;
     bool const blinn = jobs.has_material(LGPU_MAT_BLINN), film = jobs.has_material(LGPU_MAT_THINFILM);
-    wf_shade<K, J, LGPU_MAT_LAMBERTIAN, REC><<<sg, g.shade_block, 0, st>>>(jobs, wi, d_cnt);
-    // the two lists beside each other
-    cudaStream_t const fs = blinn && film ? run->fork_side(st) : st;
-    if (film) wf_shade<K, J, LGPU_MAT_THINFILM, REC><<<sg, g.shade_block, 0, fs>>>(jobs, wi, d_cnt);
-    if (fs != st) run->end_side();
-    if (blinn) wf_shade<K, J, LGPU_MAT_BLINN, REC><<<sg, g.shade_block, 0, st>>>(jobs, wi, d_cnt);
+    bool const lists = blinn || film;
+    if (!lists) {
+      wf_shade<K, J, LGPU_MAT_LAMBERTIAN, REC><<<sg, g.shade_block, 0, st>>>(jobs, wi, d_cnt);
+    } else {
+      wf_shade<K, J, kShadeRest, REC><<<sg, g.shade_block, 0, st>>>(jobs, wi, d_cnt);
+      // the lists beside each other
+      cudaStream_t const fs = run->fork_side(st);
+      if (film) wf_shade<K, J, LGPU_MAT_THINFILM, REC><<<sg, g.shade_block, 0, fs>>>(jobs, wi, d_cnt);
+      if (blinn) wf_shade<K, J, LGPU_MAT_BLINN, REC><<<sg, g.shade_block, 0, film ? st : fs>>>(jobs, wi, d_cnt);
+      run->end_side();
+      wf_shade<K, J, kShadeLamb, REC><<<sg, g.shade_block, 0, st>>>(jobs, wi, d_cnt);
+    }
     run->wait_side(st);
     run->end(2, st);
     cudaStream_t const side = run->fork_side(st);
@@ -325,7 +327,7 @@ cudaError_t wave_chunk(const J& jobs, WaveState& w, uint64_t c0, uint32_t total,
     wf_finish<K, J><<<g.fin, 256, 0, side>>>(jobs, wi, d_cnt);
     run->end_side();
     // finish, plan, shade, shadow
-    run->total += 4 + (generate ? 1 : 0) + (blinn ? 1 : 0) + (film ? 1 : 0) + closest_launches(jobs, linear);
+    run->total += 4 + (generate ? 1 : 0) + (lists ? 1 : 0) + (blinn ? 1 : 0) + (film ? 1 : 0) + closest_launches(jobs, linear);
   });
   if (e != cudaSuccess) return e;
   wf_reduce<J><<<(w.npix + 255) / 256, 256, 0, st>>>(jobs, w, c0 + total);

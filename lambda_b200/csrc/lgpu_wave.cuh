@@ -126,6 +126,7 @@ __global__ void wf_plan(WaveState w, uint32_t total) {
   w.ctl[kCtlEnded + w.par] = 0;
   w.ctl[kCtlListB] = 0;
   w.ctl[kCtlListT] = 0;
+  w.ctl[kCtlListL] = 0;
 }
 
 // Starts the planned paths at the end of the queue: work item q is sample
@@ -571,7 +572,7 @@ __global__ void __launch_bounds__(128) wf_trace_fallback(J jobs, WaveState w, De
 // a warp's lanes take the same branch of the BSDF code.  A counting sort:
 // per warp one ballot per group, a shared table of the warps' counts, and
 // each thread's rank within its group.  Returns the entry for this thread.
-constexpr int kSortGroups = 8;
+constexpr int kSortGroups = LGPU_MAT_DIREMITTER + 3;
 
 // obj_of(q) is the object that entry q hit (UINT32_MAX: none).
 template <class J, class O>
@@ -589,8 +590,10 @@ __device__ __forceinline__ uint32_t material_order(const J& jobs, const WaveStat
       key = 0;
     } else {
       const DevScene& S = jobs.scene(J::kMulti ? w.in.job[q] : 0u);
-      uint32_t const type = uint32_t(S.mats[S.objects[obj].mat].type);
-      key = 1u + (type < kSortGroups - 3 ? type : kSortGroups - 3);
+      uint32_t type = uint32_t(S.mats[S.objects[obj].mat].type);
+      // unshaded materials scatter in the Lambertian hits' code
+      if (type == LGPU_MAT_MICROFACET || type > LGPU_MAT_DIREMITTER) type = LGPU_MAT_LAMBERTIAN;
+      key = 1u + type;
     }
   }
   unsigned mine = 0;
@@ -617,11 +620,13 @@ __device__ __forceinline__ uint32_t material_order(const J& jobs, const WaveStat
 // After material_order: the block's Blinn entries are appended to the list
 // at the front of w.shade_list, its thin-film entries to the list growing
 // down from its end (both lists hold queue positions, together at most the
-// queue's length).  A group is a contiguous range of the block's threads,
-// so one atomic per list and block places it.
+// queue's length), and its Lambertian ones to w.shade_list2.  A group is a
+// contiguous range of the block's threads, so one atomic per list and block
+// places it.
 __device__ __forceinline__ void list_material_groups(const WaveState& w, uint32_t i, uint32_t group) {
-  __shared__ uint32_t lbase[2];
-  uint32_t const gb = 1u + LGPU_MAT_BLINN, gt = 1u + LGPU_MAT_THINFILM;
+  __shared__ uint32_t lbase[3];
+  uint32_t const gl = 1u + LGPU_MAT_LAMBERTIAN, gb = 1u + LGPU_MAT_BLINN, gt = 1u + LGPU_MAT_THINFILM;
+  uint32_t const below_l = uint32_t(__syncthreads_count(group < gl));
   uint32_t const below_b = uint32_t(__syncthreads_count(group < gb));
   uint32_t const cnt_b = uint32_t(__syncthreads_count(group == gb));
   uint32_t const below_t = uint32_t(__syncthreads_count(group < gt));
@@ -629,8 +634,10 @@ __device__ __forceinline__ void list_material_groups(const WaveState& w, uint32_
   if (threadIdx.x == 0) {
     lbase[0] = cnt_b ? atomicAdd(w.ctl + kCtlListB, cnt_b) : 0u;
     lbase[1] = cnt_t ? atomicAdd(w.ctl + kCtlListT, cnt_t) : 0u;
+    lbase[2] = below_b > below_l ? atomicAdd(w.ctl + kCtlListL, below_b - below_l) : 0u;
   }
   __syncthreads();
+  if (group == gl) w.shade_list2[lbase[2] + threadIdx.x - below_l] = i;
   if (group == gb) w.shade_list[lbase[0] + threadIdx.x - below_b] = i;
   if (group == gt) w.shade_list[w.cap - 1u - (lbase[1] + threadIdx.x - below_t)] = i;
   __syncthreads();  // lbase is reused by the block's next chunk
@@ -640,17 +647,63 @@ __device__ __forceinline__ void list_material_groups(const WaveState& w, uint32_
 // queued path: emitter hit (73-84), light importance sample with the MIS
 // power heuristic (87-113, its visibility left to the shadow kernel),
 // material importance sample with Russian roulette (115-143).
-// MT < 0: every path; MT = LGPU_MAT_BLINN or LGPU_MAT_THINFILM: only the
-// paths that hit that material (its code alone, the others' branches fold
-// away); MT = LGPU_MAT_LAMBERTIAN: every other path (misses, emitters,
-// Lambertian and unshaded materials).  The three specialised launches
-// together shade every path once.  REC: the primal pass of an adjoint, which
-// records what the replay reads.
+// The launches of an iteration, by what their paths hit (MT), shade every
+// path once; each has the code of its materials alone.
+//   scenes without Blinn and thin film: LGPU_MAT_LAMBERTIAN (all paths, the
+//     block's entries sorted by material);
+//   others: kShadeRest (sorts, shades misses and emitters, and lists the
+//     rest), then LGPU_MAT_BLINN, LGPU_MAT_THINFILM and kShadeLamb (Lambertian
+//     and unshaded materials) over their lists, every warp full.
+// The first kind stays for its scenes because a launch more costs them more
+// than full warps give: the 8x8 thumbnail 472 against 508 us with lists, the
+// Lambertian box room 1.85 against 1.90 ms.  The second, against one launch for
+// all but the Blinn and thin-film lists: benchmark frame 277.2 -> 270.2 ms
+// (39.1 ms of shading become 10.8 + 21.5), mixed materials 8.18 -> 7.78 ms.
+// Without scattering code kShadeRest fits 6 blocks of 256 threads on an SM
+// (4 blocks for the others): 10.8 ms against 14.0 with 8 and 11.9 with 5.
+// REC: the primal pass of an adjoint, which records what the replay reads.
+constexpr int kShadeLamb = 10, kShadeRest = 11;
+template <int MT>
+constexpr bool kShadeLists = MT == LGPU_MAT_BLINN || MT == LGPU_MAT_THINFILM || MT == kShadeLamb;
 template <int MT>
 __device__ __forceinline__ bool shade_group(uint32_t group) {
-  if (MT < 0) return true;
-  if (MT == LGPU_MAT_BLINN || MT == LGPU_MAT_THINFILM) return group == 1u + MT;
-  return group != 1u + LGPU_MAT_BLINN && group != 1u + LGPU_MAT_THINFILM;
+  return MT != kShadeRest || group < 1u + LGPU_MAT_LAMBERTIAN || group > 1u + LGPU_MAT_THINFILM;
+}
+// Entry j of a list launch (UINT32_MAX past its end) and the list's length.
+template <int MT>
+__device__ __forceinline__ uint32_t shade_list_length(const WaveState& w) {
+  return w.ctl[MT == LGPU_MAT_BLINN ? kCtlListB : (MT == LGPU_MAT_THINFILM ? kCtlListT : kCtlListL)];
+}
+template <int MT>
+__device__ __forceinline__ uint32_t shade_list_entry(const WaveState& w, uint32_t j, uint32_t n) {
+  if (j >= n) return UINT32_MAX;
+  if (MT == kShadeLamb) return w.shade_list2[j];
+  return w.shade_list[MT == LGPU_MAT_BLINN ? j : w.cap - 1u - j];
+}
+// A material as a launch sees it: the types it cannot meet are ruled out for
+// the compiler.
+template <int MT>
+__device__ __forceinline__ DevMaterial shade_material(const DevScene& S, uint32_t idx) {
+  DevMaterial x = S.mats[idx];
+  if (MT == LGPU_MAT_BLINN || MT == LGPU_MAT_THINFILM) x.type = MT;
+  if (MT == kShadeLamb) x.type = x.type == LGPU_MAT_LAMBERTIAN ? LGPU_MAT_LAMBERTIAN : LGPU_MAT_MICROFACET;
+  if (MT == kShadeRest) x.type = x.type == LGPU_MAT_DIREMITTER ? LGPU_MAT_DIREMITTER : LGPU_MAT_EMITTER;
+  if (MT == LGPU_MAT_LAMBERTIAN && (x.type == LGPU_MAT_BLINN || x.type == LGPU_MAT_THINFILM))
+    x.type = LGPU_MAT_MICROFACET;
+  return x;
+}
+// What a launch's materials leave of the BSDF cases and lobes.
+template <int MT>
+__device__ __forceinline__ void shade_cases(BsdfScalars& bl, MatSample& ms) {
+  if (MT == LGPU_MAT_LAMBERTIAN || MT == kShadeLamb) {
+    bl.kind = bl.kind ? 1 : 0;
+    ms.lobe = ms.lobe ? 1 : 0;
+  } else if (MT == LGPU_MAT_BLINN) {
+    bl.kind = bl.kind == 2 ? 2 : 3;
+  } else if (MT == LGPU_MAT_THINFILM) {
+    bl.kind = bl.kind ? 4 : 0;
+    ms.lobe = ms.lobe ? 4 : 0;
+  }
 }
 
 // Bound by memory latency (35 % of the issue slots, 2.4 TB/s of path state)
@@ -660,34 +713,26 @@ __device__ __forceinline__ bool shade_group(uint32_t group) {
 // 16-byte words of four wavelengths but computes one at a time: unrolled by
 // four, its code overflowed the instruction cache (8 of 23 stalls) and was
 // 17 % slower than 4-byte accesses.  4 blocks of 256 per SM (64 registers)
-// for the first launch and the lists: 5 are 2 % faster on the benchmark
-// frame's first launch but 7 % slower on the box room's; 6 and 5 before.
-// Benchmark frame: first launch 48.2 -> 39.2 ms, Blinn list 16.5 -> 14.9,
-// thin-film list 16.3 -> 14.3; box room 605 -> 472 us.
+// where scattering is evaluated: 5 are 2 % faster for the benchmark frame's
+// Lambertian hits but 7 % slower for the box room; 6 and 5 before.
+// Benchmark frame: misses, emitters and Lambertian hits 48.2 -> 32.3 ms, Blinn
+// list 16.5 -> 14.9, thin-film list 16.3 -> 14.3; box room 605 -> 472 us.
 template <int K, class J, int MT, bool REC>
-__global__ void __launch_bounds__(kMaxShadeBlock, 4) wf_shade(J jobs, WaveState w, DevCounters* cnt) {
+__global__ void __launch_bounds__(kMaxShadeBlock, MT == kShadeRest ? 6 : 4) wf_shade(J jobs, WaveState w, DevCounters* cnt) {
   uint32_t const n = *w.n_in;
   uint32_t const cap = w.cap;
   PathBuf const& in = w.in;
   PathBuf const& out = w.out;
   enum : int { kEnd = 0, kEmit = 1, kScatter = 2 };
-  // the Blinn and thin-film launches run over their lists (dense warps)
-  constexpr bool kList = MT == LGPU_MAT_BLINN || MT == LGPU_MAT_THINFILM;
-  uint32_t const n_loop = kList ? w.ctl[MT == LGPU_MAT_BLINN ? kCtlListB : kCtlListT] : n;
+  constexpr bool kList = kShadeLists<MT>;
+  uint32_t const n_loop = kList ? shade_list_length<MT>(w) : n;
   for (uint32_t base = blockIdx.x * blockDim.x; base < n_loop; base += gridDim.x * blockDim.x) {
-    uint32_t group = 0;
-    // the first launch sorts each block's entries by material and appends
-    // the Blinn and thin-film ones to the lists of the other two launches,
-    // which shade them with full warps instead of the quarter of each block
-    // that has their material (shading -24 % measured)
-    uint32_t i;
+    uint32_t group = 0, i;
     if (kList) {
-      uint32_t const j = base + threadIdx.x;
-      i = j < n_loop ? w.shade_list[MT == LGPU_MAT_BLINN ? j : cap - 1u - j] : UINT32_MAX;
-      group = 1u + MT;
+      i = shade_list_entry<MT>(w, base + threadIdx.x, n_loop);
     } else {
       i = material_order(jobs, w, base, n, &group, [&](uint32_t q) { return w.hobj[q]; });
-      if (MT == LGPU_MAT_LAMBERTIAN) list_material_groups(w, i, group);
+      if (MT == kShadeRest) list_material_groups(w, i, group);
     }
     bool const live = i < n && shade_group<MT>(group);
     uint32_t const jb = (J::kMulti && live) ? in.job[i] : 0u;
@@ -695,16 +740,7 @@ __global__ void __launch_bounds__(kMaxShadeBlock, 4) wf_shade(J jobs, WaveState 
     const RenderArgs& a = jobs.args(jb);
     float const omega = S.lambda_sup - S.lambda_inf;
     float const step = omega / float(K);
-    // the material as this launch sees it: a specialised launch knows its
-    // type at compile time
-    auto material = [&](uint32_t idx) {
-      DevMaterial x = S.mats[idx];
-      if (kList) x.type = MT;
-      // neither Blinn nor thin film (the compiler then drops their code)
-      if (MT == LGPU_MAT_LAMBERTIAN && (x.type == LGPU_MAT_BLINN || x.type == LGPU_MAT_THINFILM))
-        x.type = LGPU_MAT_MICROFACET;
-      return x;
-    };
+    auto material = [&](uint32_t idx) { return shade_material<MT>(S, idx); };
     int kind = kEnd;
     bool cont = false, shadow = false, needs_test = false;
     f3 sp = f3{0.f, 0.f, 0.f}, sd = f3{0.f, 0.f, 1.f};
@@ -783,16 +819,7 @@ __global__ void __launch_bounds__(kMaxShadeBlock, 4) wf_shade(J jobs, WaveState 
         }
       }
     }
-    // what this launch's materials leave of the BSDF cases and lobes
-    if (MT == LGPU_MAT_LAMBERTIAN) {
-      bl.kind = bl.kind ? 1 : 0;
-      ms.lobe = ms.lobe ? 1 : 0;
-    } else if (MT == LGPU_MAT_BLINN) {
-      bl.kind = bl.kind == 2 ? 2 : 3;
-    } else if (MT == LGPU_MAT_THINFILM) {
-      bl.kind = bl.kind ? 4 : 0;
-      ms.lobe = ms.lobe ? 4 : 0;
-    }
+    shade_cases<MT>(bl, ms);
     // compacted appends: next queue, ended list, shadow queue
     bool const ended = live && !cont;
     uint32_t const o_pos = warp_append(w.n_out, cont);
