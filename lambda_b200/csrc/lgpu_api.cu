@@ -93,6 +93,7 @@ struct lgpu_ctx {
   DevArray<uint32_t> job_pixels;
   DevArray<float> batch_out;
   DevArray<float> adj_buf;
+  DevArray<double> adj_sums;
   // working buffers
   DevArray<float> out;
   // wavefront state (lgpu_wave.cuh), sized for the largest frame rendered
@@ -587,10 +588,12 @@ int adjoint_impl(lgpu_ctx* ctx, const lgpu_render_params* p, const float* d_dimg
   if (int r = ensure_wave(ctx, a.pixel_count, n_items, chunk, false, ws, true, false, record)) return r;
   if (int r = prepare_launch(ctx, (p->flags & LGPU_FLAG_KERNEL_TIMING) != 0)) return r;
   size_t const n_spec = ctx->slots[0].spectra.n;
-  cudaError_t e = cudaMemsetAsync(ctx->counters, 0, 3 * sizeof(DevCounters), st);
+  cudaError_t e = ensure(ctx->adj_sums, 2 * size_t(S.n_materials));
+  if (e == cudaSuccess) e = cudaMemsetAsync(ctx->counters, 0, 3 * sizeof(DevCounters), st);
   if (e == cudaSuccess) e = cudaMemsetAsync(d_gspec, 0, n_spec * sizeof(float), st);
-  if (e == cudaSuccess) e = cudaMemsetAsync(d_gmat, 0, 4 * size_t(S.n_materials) * sizeof(float), st);
-  AdjointArgs const g{d_dimg, d_gspec, d_gmat};
+  if (e == cudaSuccess)
+    e = cudaMemsetAsync(ctx->adj_sums.ptr, 0, 2 * size_t(S.n_materials) * sizeof(double), st);
+  AdjointArgs const g{d_dimg, d_gspec, d_gmat, ctx->adj_sums.ptr};
   if (e == cudaSuccess) e = cudaEventRecord(ctx->ev0, st);
   if (e == cudaSuccess) e = launch_adjoint(S.hero_k, S, a, &ws, chunk, d_img, g, ctx->counters, st, &ctx->launch);
   if (e == cudaSuccess) e = cudaEventRecord(ctx->ev1, st);
@@ -927,6 +930,7 @@ void lgpu_destroy(lgpu_ctx* ctx) {
   ctx->job_pixels.release();
   ctx->batch_out.release();
   ctx->adj_buf.release();
+  ctx->adj_sums.release();
   if (ctx->h_ctl) cudaFreeHost(ctx->h_ctl);
   ctx->rays.release();
   ctx->hits.release();

@@ -335,6 +335,7 @@ struct AdjointArgs {
   const float* dimg;  // dLoss/d(linear RGB), width*height*3, row 0 at the top
   float* g_spec;      // n_spectra * n_bins
   float* g_mat;       // n_materials * 4: thickness, alpha, 0, 0
+  double* g_mat_sum;  // n_materials * 2, zeroed: thickness, alpha
 };
 cudaError_t launch_adjoint(uint32_t hero_k, const DevScene& S, const RenderArgs& a, WaveState* wave,
                            uint64_t chunk_items, float* d_img, const AdjointArgs& g, DevCounters* d_cnt,
