@@ -272,6 +272,20 @@ cudaError_t run_iterations(WaveState& w, uint32_t total, uint32_t max_scatter, c
   }
 }
 
+// Blocks of a list launch for a queue of sg blocks.  A list's length is known
+// on the device only; blocks past it cost their launch and one read, blocks
+// short of it a loop whose rounds wait for their slowest warp.  A quarter of
+// the queue, but 16 blocks per SM (four rounds of them) at least: against a
+// full grid benchmark frame 270.5 -> 267.9 ms, 4K frame in tiles 33.6 -> 32.6,
+// 9 instances at 1021x577 8.29 -> 8.12, and a frame whose hits are all of one
+// list 12.14 -> 12.12 ms; 4 blocks per SM at least cost the benchmark frame 276
+// ms, no least number an inverse step 3.88 -> 4.05 ms.  The adjoint's launches
+// keep the full grid (26.05 ms with a quarter, 25.77).
+inline uint32_t list_grid(uint32_t sg, uint32_t sms) {
+  uint32_t const quarter = (sg + 3) / 4, few = 16u * sms;
+  return quarter > few ? quarter : (sg < few ? sg : few);
+}
+
 // One chunk of the streaming wavefront: work items [c0, c0 + total).
 // Every iteration appends new paths behind the queue up to its capacity
 // (plan + generate), advances every queued path by one segment (trace, shade,
@@ -311,11 +325,12 @@ cudaError_t wave_chunk(const J& jobs, WaveState& w, uint64_t c0, uint32_t total,
     } else {
       wf_shade<K, J, kShadeRest, REC><<<sg, g.shade_block, 0, st>>>(jobs, wi, d_cnt);
       // the lists beside each other
+      uint32_t const lg = REC ? sg : list_grid(sg, wave_occupancy<K, J>().sms);
       cudaStream_t const fs = run->fork_side(st);
-      if (film) wf_shade<K, J, LGPU_MAT_THINFILM, REC><<<sg, g.shade_block, 0, fs>>>(jobs, wi, d_cnt);
-      if (blinn) wf_shade<K, J, LGPU_MAT_BLINN, REC><<<sg, g.shade_block, 0, film ? st : fs>>>(jobs, wi, d_cnt);
+      if (film) wf_shade<K, J, LGPU_MAT_THINFILM, REC><<<lg, g.shade_block, 0, fs>>>(jobs, wi, d_cnt);
+      if (blinn) wf_shade<K, J, LGPU_MAT_BLINN, REC><<<lg, g.shade_block, 0, film ? st : fs>>>(jobs, wi, d_cnt);
       run->end_side();
-      wf_shade<K, J, kShadeLamb, REC><<<sg, g.shade_block, 0, st>>>(jobs, wi, d_cnt);
+      wf_shade<K, J, kShadeLamb, REC><<<lg, g.shade_block, 0, st>>>(jobs, wi, d_cnt);
     }
     run->wait_side(st);
     run->end(2, st);

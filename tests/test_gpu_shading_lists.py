@@ -61,3 +61,23 @@ def test_same_image(scenes, width, unshaded, extra):
     for a, b in zip(*grads):
         na, nb = (np.linalg.norm(x.astype(np.float64)) for x in (a, b))
         assert np.isfinite(na) and abs(na - nb) <= 2e-5 * nb
+
+
+def test_list_longer_than_its_grid(tmp_path):
+    """2^21 paths: the list's launch has 16 blocks of 256 per SM, a third of
+    its hits."""
+    from lambda_b200.renderer import Context
+    from lambda_b200.scene import load_nls
+    nls = synth.box_room(str(tmp_path), width=1024)
+    with open(nls) as f:
+        j = json.load(f)
+    images = []
+    for name in ("none", "blinn"):
+        path = os.path.join(str(tmp_path), name + ".nls")
+        with open(path, "w") as f:
+            json.dump(dict(j, materials=j["materials"] + ([EXTRA[name]] if name in EXTRA else [])), f)
+        ctx = Context(0)
+        ctx.upload(load_nls(path))
+        images.append(ctx.render(2, 4, 0.85, seed=4))
+        ctx.close()
+    assert np.array_equal(images[0].view(np.uint32), images[1].view(np.uint32))
