@@ -427,7 +427,7 @@ cudaError_t replay_chunk(const OneJob& jobs, WaveState& w, uint64_t c0, uint32_t
       run->begin(0, st);
       launch_closest<K>(jobs, wi, gr, linear, c_closest, st);
       run->end(0, st);
-      run->total += closest_launches(jobs, linear);
+      run->total += closest_launches(linear);
     }
     run->begin(2, st);
     // one block per queue chunk (see wave_chunk)

@@ -159,15 +159,12 @@ void launch_closest(const J& jobs, const WaveState& w, const WaveGrids& g, bool 
     wf_trace<J><<<g.trace, 128, kTraceSmem, st>>>(jobs, w, cnt);
   } else {
     wf_trace_persistent<false, K, J><<<g.ptrace, 128, kTraceSmem, st>>>(jobs, w, cnt);
-    if (jobs.max_objects() > kMaxLoopObjects) wf_trace_fallback<J><<<g.fb, 128, 0, st>>>(jobs, w, cnt);
+    wf_trace_fallback<J><<<g.fb, 128, 0, st>>>(jobs, w, cnt);
   }
 }
 
 // Kernel launches of launch_closest.
-template <class J>
-uint32_t closest_launches(const J& jobs, bool linear) {
-  return !linear && jobs.max_objects() > kMaxLoopObjects ? 2 : 1;
-}
+inline uint32_t closest_launches(bool linear) { return linear ? 1 : 2; }
 
 // Swaps the current and next queue, and the shadow contributions of this
 // and the last iteration, after an iteration.
@@ -342,7 +339,7 @@ cudaError_t wave_chunk(const J& jobs, WaveState& w, uint64_t c0, uint32_t total,
     wf_finish<K, J><<<g.fin, 256, 0, side>>>(jobs, wi, d_cnt);
     run->end_side();
     // finish, plan, shade, shadow
-    run->total += 4 + (generate ? 1 : 0) + (lists ? 1 : 0) + (blinn ? 1 : 0) + (film ? 1 : 0) + closest_launches(jobs, linear);
+    run->total += 4 + (generate ? 1 : 0) + (lists ? 1 : 0) + (blinn ? 1 : 0) + (film ? 1 : 0) + closest_launches(linear);
   });
   if (e != cudaSuccess) return e;
   wf_reduce<J><<<(w.npix + 255) / 256, 256, 0, st>>>(jobs, w, c0 + total);

@@ -4,7 +4,7 @@
 // The rays of a query are put into a wavefront queue (closest-hit queries)
 // or the shadow-ray queue (any-hit queries) of a WaveState of their own and
 // traced by exactly the kernels a render launches for them:
-// wf_trace_persistent<false> (+ wf_trace_fallback; instance BVH) or wf_trace
+// wf_trace_persistent<false> + wf_trace_fallback (instance BVH) or wf_trace
 // (the reference's linear object loop) for closest hits, and
 // wf_trace_persistent<true> or wf_shadow for shadow rays.  The hit records
 // are then expanded to lgpu_hit with the same finalize_hit the shading uses.
@@ -102,7 +102,7 @@ TraceGrids trace_grids(const WaveConfig& cfg) {
 uint32_t trace_launches(const DevScene& S, bool any, uint32_t flags) {
   bool const linear = (flags & LGPU_FLAG_REFERENCE_ORDER) || S.n_objects <= 4;
   // setup, load, store and the traversal
-  return 4 + (!any && !linear && S.n_objects > kMaxLoopObjects ? 1 : 0);
+  return 4 + (!any && !linear ? 1 : 0);
 }
 
 size_t trace_wave_layout(uint8_t* base, uint32_t cap, WaveState& ws) {
@@ -151,7 +151,7 @@ cudaError_t launch_trace_chunk(const DevScene& S, WaveState& w, const float* d_r
       wf_trace<OneJob><<<g.trace, 128, kTraceSmem, st>>>(jobs, w, d_cnt);
     } else {
       wf_trace_persistent<false, 16, OneJob><<<g.ptrace, 128, kTraceSmem, st>>>(jobs, w, d_cnt);
-      if (S.n_objects > kMaxLoopObjects) wf_trace_fallback<OneJob><<<g.fb, 128, 0, st>>>(jobs, w, d_cnt);
+      wf_trace_fallback<OneJob><<<g.fb, 128, 0, st>>>(jobs, w, d_cnt);
     }
     trace_store<<<(n + 127) / 128, 128, 0, st>>>(S, w, n, d_hits);
   } else {

@@ -73,15 +73,6 @@ struct SplitStack {
 };
 
 constexpr int kSplitCap = kSmemStack + kLocalStack;
-// Scenes whose order-dependent rays run the reference's object loop inside
-// the closest-hit kernel (phase 4): its object groups and a mesh's entries
-// fit the stack together.  Beyond that, wf_trace_fallback runs it.  A second
-// launch costs the latency of one such ray behind every closest-hit launch
-// (14 box rooms with instances, 20 iterations: closest-hit 4.8 + 1.3 ms with
-// it, 5.3 ms without; box room 0.87 + 0.12 against 0.93 ms).
-constexpr uint32_t kMaxLoopObjects = 1024;
-static_assert(kMaxLoopObjects / 32 + kStackCap <= kSplitCap, "object groups and a mesh's entries");
-
 // push_children (lgpu_intersect.cuh) writing through a SplitStack.  With
 // `sorted` false (any-hit queries, whose boolean answer does not depend on
 // the visiting order) the hit children are pushed in child order.
@@ -368,8 +359,7 @@ __device__ __forceinline__ void node_children(const WideNode& nd, const Ray& r, 
 // A stack entry is a child reference with its entry distance, or, with
 // kGroupBit set, a node some of whose hit children were not visited yet:
 // their mask in the 8 low bits of t, whose other bits are a lower bound of
-// their entry distances.  In phase 4 a group entry in world space is 32
-// objects from an index on, with the mask of those still to be tested in t.
+// their entry distances.
 constexpr uint32_t kGroupBit = 0x40000000u;  // node indices stay below it (kMaxSlots)
 constexpr uint32_t kNoRef = kEmptyChild;
 
@@ -410,12 +400,10 @@ struct TraceState {
   int base;        // stack height at which the entered mesh is done; -1 in world space
   bool lowered;    // z was lowered for the entered mesh (it loses ties)
   // 1: closest hit; 2: any hit among the objects below wobj; 3: closest hit
-  // without object wobj; 4: the reference's loop over the objects in index
-  // order, through its trees (any-hit kernels: 1, any hit without object wobj)
+  // without object wobj (any-hit kernels: 1, any hit without object wobj)
   int phase;
-  uint32_t wobj;  // with kOthersInside: more than one mesh's bounds contain the ray origin
+  uint32_t wobj;
 };
-constexpr uint32_t kOthersInside = 0x80000000u;
 
 // The next step: node or leaf `ref`, or the stack's top if it is kNoRef.
 __device__ __forceinline__ void trace_next(TraceState& t, uint32_t ref) {
@@ -465,10 +453,6 @@ __device__ __forceinline__ void trace_pop(const DevScene& S, TraceState& t, Spli
       if (rest) st.push(StackEntry{ref, __uint_as_float(rest)});
       ref = S.nodes[ref ^ kGroupBit].child[c];
     }
-  } else if (t.phase == 4 && t.base < 0) {
-    uint32_t const m = __float_as_uint(e.t), rest = m & (m - 1u);
-    if (rest) st.push(StackEntry{ref, __uint_as_float(rest)});
-    ref = kLeafBit | ((ref ^ kGroupBit) + uint32_t(__ffs(m) - 1));
   } else {
     if (e.t > t.z * kTravSlack) return;
     if (!(ref & kLeafBit) && (ref & kGroupBit)) {
@@ -593,7 +577,7 @@ __device__ __forceinline__ void trace_object(const DevScene& S, TraceState& t, S
   uint32_t const cnt = ((t.ref >> 28) & 7u) + 1u;
   uint32_t const slot = t.ref & kSlotMask;
   t.kind = kLanePop;
-  uint32_t const i = (!ANY && t.phase == 4) ? slot : S.tlas_objects[slot];
+  uint32_t const i = S.tlas_objects[slot];
   if (cnt > 1) {
     if (st.sp + 1 > kSplitCap) {
       st.flags |= kTravOverflow;
@@ -602,7 +586,7 @@ __device__ __forceinline__ void trace_object(const DevScene& S, TraceState& t, S
     }
     st.push(StackEntry{kLeafBit | ((cnt - 2u) << 28) | (slot + 1u), 0.f});
   }
-  if (ANY ? i == t.wobj : ((t.phase == 2 && i >= (t.wobj & ~kOthersInside)) || (t.phase == 3 && i == t.wobj))) return;
+  if (ANY ? i == t.wobj : ((t.phase == 2 && i >= t.wobj) || (t.phase == 3 && i == t.wobj))) return;
   insts++;
   const DevObject& ob = S.objects[i];
   bool const low = !any && t.obj != UINT32_MAX && i < t.obj;
@@ -636,9 +620,9 @@ __device__ __forceinline__ void trace_object(const DevScene& S, TraceState& t, S
   float ex;
   float r0 = aabb_scalar(m.bounds, li, z, inside, ex);
   if (!ANY && r0 != kFltMax && inside) t.n_inside++;
-  // only the reference's loop and shadow rays enter a mesh from inside at its
-  // exit distance
-  if (!ANY && t.phase != 4 && r0 != kFltMax && inside) r0 = kBias;
+  // only shadow rays (and the reference's loop) enter a mesh from inside at
+  // its exit distance
+  if (!ANY && r0 != kFltMax && inside) r0 = kBias;
   if (r0 == kFltMax || r0 > z) return;
   st.ws[0] = t.w.p.x;
   st.ws[128] = t.w.p.y;
@@ -655,7 +639,7 @@ __device__ __forceinline__ void trace_object(const DevScene& S, TraceState& t, S
   t.cur_exit = inside ? ex : -1.f;
   t.lowered = low;
   t.base = st.sp;
-  trace_next(t, (!ANY && t.phase == 4) ? m.root : m.trav_root);
+  trace_next(t, m.trav_root);
 }
 
 // intersect::scene for the wavefront kernels: the instance BVH through

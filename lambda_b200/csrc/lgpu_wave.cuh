@@ -407,7 +407,6 @@ __global__ void __launch_bounds__(128, ANY ? 7 : 6) wf_trace_persistent(J jobs, 
     uint32_t const sum = __reduce_add_sync(FULL, t.kind);
     int const n_tri = int((sum >> 8) & 0xFFu), n_obj = int((sum >> 16) & 0xFFu);
     if (int((sum >> 24) & 0x3Fu) >= wait) {
-      bool loop = false;
       if (t.kind == kLaneDone) {
         t.kind = kLaneIdle;
         if (ANY) {
@@ -416,61 +415,34 @@ __global__ void __launch_bounds__(128, ANY ? 7 : 6) wf_trace_persistent(J jobs, 
           // The winner W of phase 1 may be a mesh whose bounds contain the ray
           // origin and which the ray leaves after the hit.  The reference
           // skips W if an object tested before it (lower index) was hit before
-          // that exit (cg.hpp:1393, 1414).  An any-hit query over the
-          // lower-index objects up to the exit (phase 2; nothing to ask for
-          // object 0) decides most rays: without a hit W stands.  With one,
-          // the answer is the closest hit without W (phase 3) if W is the only
-          // such mesh; if there are more, whether each counts depends on the
-          // others, and the reference's loop is run (phase 4).  Asking first
-          // also when there are more leaves 1 in 50 to 120 of those rays for
-          // the loop (box room 90,612 -> 728 of 3.7 M rays, its closest hits
-          // 1.15 -> 0.93 ms a frame; 14 box rooms with instances 207,678 ->
-          // 4,420, frame 13.1 -> 10.9 ms).
-          bool const ask = t.phase == 1 && t.exit > t.z && t.obj != 0u, again = t.phase == 2 && t.obj != UINT32_MAX;
+          // that exit (cg.hpp:1393, 1414).  If W is the only such mesh, an
+          // any-hit query over the lower-index objects up to the exit (phase
+          // 2; nothing to ask for object 0) decides it: without a hit W
+          // stands, with one the answer is the closest hit without W (phase
+          // 3).  If there are more, whether each counts depends on the
+          // others, and the reference's loop answers (wf_trace_fallback).
+          //
+          // Asking first in that case too would leave 1 in 50 to 120 of those
+          // rays for the loop (box room 1.86 instead of 2.08 ms, 14 box rooms
+          // with instances 8.9 instead of 11.3 ms), but gives other answers:
+          // the loop's exact box tests in the reference's trees reject
+          // triangles that a ray grazes and that this search finds (one batch
+          // in 75 of such rooms had a different image).
+          bool const order = t.phase == 1 && t.exit > t.z, alone = t.n_inside == 1;
+          bool const ask = order && alone && t.obj != 0u, again = t.phase == 2 && t.obj != UINT32_MAX;
+          if (order && !alone) w.fb_queue[atomicAdd(w.ctl + kCtlFallback, 1u)] = idx;
           if (t.phase != 2) w.hobj[idx] = t.obj;
           if (ask || again) {
             t.w = load_ray(w.in.ra, w.in.rb, idx);
-            uint32_t const others = t.n_inside;
             if (ask) {
               t.z = prev_float(t.exit);
               t.wobj = t.obj;
               t.phase = 2;
-              if (others != 1) t.wobj |= kOthersInside;
             } else {
               t.z = kFltMax;
-              t.phase = (t.wobj & kOthersInside) ? 4 : 3;
+              t.phase = 3;
             }
             trace_begin(jobs.scene(jb), t, st);
-            if (t.phase == 4) {
-              if (jobs.scene(jb).n_objects <= kMaxLoopObjects) {
-                t.kind = kLanePop;
-                loop = true;
-              } else {
-                t.kind = kLaneIdle;
-                w.fb_queue[atomicAdd(w.ctl + kCtlFallback, 1u)] = idx;
-              }
-            }
-          }
-        }
-      }
-      // Rays for the object loop: the warp drops, 32 at a time, the objects a
-      // ray cannot hit at any distance (every test of the loop only gets
-      // stricter as the distance bound shrinks); the others wait on the stack
-      // of the ray's lane, the lowest indices on top.
-      if (!ANY) {
-        unsigned const loops = __ballot_sync(FULL, loop);
-        if (loops && lane == 0) atomicAdd(&cnt->ordered, static_cast<unsigned long long>(__popc(loops)));
-        for (unsigned m = loops; m; m &= m - 1u) {
-          int const src = __ffs(m) - 1;
-          const DevScene& S = jobs.scene(__shfl_sync(FULL, jb, src));
-          Ray r;
-          r.p = f3{__shfl_sync(FULL, t.w.p.x, src), __shfl_sync(FULL, t.w.p.y, src), __shfl_sync(FULL, t.w.p.z, src)};
-          r.u = f3{__shfl_sync(FULL, t.w.u.x, src), __shfl_sync(FULL, t.w.u.y, src), __shfl_sync(FULL, t.w.u.z, src)};
-          r.inv = f3{0.f, 0.f, 0.f};  // the tests below use the local rays' own
-          for (uint32_t b = (S.n_objects + 31u) / 32u; b-- > 0u;) {
-            uint32_t const o = 32u * b + uint32_t(lane);
-            unsigned const may = __ballot_sync(FULL, o < S.n_objects && object_may_hit(S, o, r));
-            if (lane == src && may) st.push(StackEntry{kGroupBit | (32u * b), __uint_as_float(may)});
           }
         }
       }
@@ -522,8 +494,7 @@ __global__ void __launch_bounds__(128, ANY ? 7 : 6) wf_trace_persistent(J jobs, 
 }
 
 // Extension rays whose closest hit depends on the reference's object order
-// (see scene_hit) in scenes of more than kMaxLoopObjects objects: the linear
-// object loop, one warp per ray.  The lanes
+// (see scene_hit): the linear object loop, one warp per ray.  The lanes
 // first test 32 objects at a time with an unbounded distance (the objects
 // the ray cannot hit at all drop out); lane 0 then runs the reference's
 // loop over the remaining ones in index order.  A launch has few such rays
