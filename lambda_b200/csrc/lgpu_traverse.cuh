@@ -454,11 +454,15 @@ __device__ __forceinline__ void trace_pop(const DevScene& S, TraceState& t, Spli
       ref = S.nodes[ref ^ kGroupBit].child[c];
     }
   } else {
-    if (e.t > t.z * kTravSlack) return;
+    uint32_t bound = __float_as_uint(e.t);
     if (!(ref & kLeafBit) && (ref & kGroupBit)) {
-      todo = __float_as_uint(e.t) & 0xFFu;
+      // without the mask, which would lift the bound by up to 252 units in
+      // the last place, over the slack's 128 to 256
+      todo = bound & 0xFFu;
+      bound &= ~0xFFu;
       ref ^= kGroupBit;
     }
+    if (__uint_as_float(bound) > t.z * kTravSlack) return;
   }
   trace_next(t, ref);
 }
