@@ -119,6 +119,7 @@ struct lgpu_ctx {
   cudaEvent_t ev_fork = nullptr, ev_join = nullptr;
   cudaStream_t beside = nullptr;  // the wavefront's shadow and film launches
   cudaEvent_t ev_bfork = nullptr, ev_bjoin = nullptr;
+  cudaEvent_t ev_asked[2] = {nullptr, nullptr};
   cudaStream_t side = nullptr;  // batches: the megakernel jobs
   bool keep_counters = false;   // the counters were reset by the caller of a nested render
 
@@ -348,6 +349,7 @@ int prepare_launch(lgpu_ctx* ctx, bool timing) {
   ctx->launch.side = ctx->beside;
   ctx->launch.fork = ctx->ev_bfork;
   ctx->launch.join = ctx->ev_bjoin;
+  for (int k = 0; k < 2; k++) ctx->launch.asked[k] = ctx->ev_asked[k];
   return LGPU_OK;
 }
 
@@ -907,8 +909,10 @@ int lgpu_create(int device, lgpu_ctx** out) {
   if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&ctx->beside, cudaStreamNonBlocking);
   if (e == cudaSuccess) e = cudaEventCreateWithFlags(&ctx->ev_bfork, cudaEventDisableTiming);
   if (e == cudaSuccess) e = cudaEventCreateWithFlags(&ctx->ev_bjoin, cudaEventDisableTiming);
+  for (cudaEvent_t& ev : ctx->ev_asked)
+    if (e == cudaSuccess) e = cudaEventCreateWithFlags(&ev, cudaEventDisableTiming);
   if (e == cudaSuccess) e = cudaMalloc(&ctx->counters, 3 * sizeof(DevCounters));
-  if (e == cudaSuccess) e = cudaMallocHost(&ctx->h_ctl, kCtlWords * sizeof(uint32_t));
+  if (e == cudaSuccess) e = cudaMallocHost(&ctx->h_ctl, (kCtlWords + 2) * sizeof(uint32_t));
   if (e != cudaSuccess) {
     lgpu_destroy(ctx);
     return e == cudaErrorMemoryAllocation ? LGPU_ERR_OUT_OF_MEMORY : LGPU_ERR_CUDA;
@@ -956,6 +960,8 @@ void lgpu_destroy(lgpu_ctx* ctx) {
   }
   if (ctx->ev_bfork) cudaEventDestroy(ctx->ev_bfork);
   if (ctx->ev_bjoin) cudaEventDestroy(ctx->ev_bjoin);
+  for (cudaEvent_t ev : ctx->ev_asked)
+    if (ev) cudaEventDestroy(ev);
   ctx->graph.release();
   for (auto& k : ctx->launch.ev)
     for (auto& s : k)

@@ -83,7 +83,7 @@ struct WaveState {
                          // of the thin-film hits (from the back), for their shading launches
   uint32_t* shade_list2; // cap: of the Lambertian and unshaded hits
   uint32_t* ctl;       // kCtlWords counters
-  uint32_t* h_ctl;     // pinned host copy of ctl
+  uint32_t* h_ctl;     // pinned host copy of ctl, and of two queue lengths behind it
   float* sbuf;         // 3 per work item of a chunk: XYZ of every (sample, pixel)
   float* film;         // 3*npix XYZ
   double* film64;      // 3*npix XYZ in double (LGPU_FLAG_FP64_FILM), or nullptr
@@ -156,6 +156,7 @@ struct WaveLaunch {
   // the stream of the shadow and film launches and its fork and join events
   cudaStream_t side = nullptr;
   cudaEvent_t fork = nullptr, join = nullptr;
+  cudaEvent_t asked[2] = {nullptr, nullptr};  // queue-length readbacks of two pairs of iterations
   bool forked = false;  // side work that st does not wait for yet
   unsigned long long graph_launches = 0;
   bool on = false;
