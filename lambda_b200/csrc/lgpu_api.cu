@@ -314,6 +314,18 @@ int ensure_wave(lgpu_ctx* ctx, uint32_t npix, uint64_t n_items, uint64_t chunk_i
   uint64_t const qcap = ctx->cfg.queue_cap ? ctx->cfg.queue_cap : kQueueCap;
   uint32_t const cap = uint32_t(n_items < qcap ? n_items : qcap);
   size_t bytes = wave_layout(nullptr, cap, K, npix, chunk_items, batch, adjoint, fp64, record, ws);
+  if (record && bytes > ctx->w_arena.cap) {
+    // the hits take at most half of the memory that the rest of the arena
+    // leaves, so that a program's own allocations still fit
+    size_t const rest = wave_layout(nullptr, cap, K, npix, chunk_items, batch, adjoint, fp64, 0, ws);
+    size_t free = 0, all = 0;
+    cudaError_t const q = cudaMemGetInfo(&free, &all);
+    if (q != cudaSuccess) return cuda_fail(ctx, q, "free memory");
+    if (rest + 2 * (bytes - rest) > free + ctx->w_arena.cap) {
+      record = 0;
+      bytes = rest;
+    }
+  }
   cudaError_t e = ensure(ctx->w_arena, bytes);
   if (e == cudaErrorMemoryAllocation && record) {
     // without room for the hits, the replay traces its rays
