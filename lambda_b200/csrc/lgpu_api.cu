@@ -591,10 +591,11 @@ int adjoint_impl(lgpu_ctx* ctx, const lgpu_render_params* p, const float* d_dimg
   uint64_t const max_items = (uint64_t(1) << 34) / per_item;
   uint64_t const chunk = n_items < max_items ? n_items : max_items;
   // the primal pass keeps the hits of its vertices for the replay (4 + 32 B
-  // each, max_scatterings + 2 per item) while they take at most 8 GiB: the
-  // replay then traces no rays (512x512, 32 spp, 4 bounces: 10.6 of 38 ms).
-  // More would not fit beside other work on the device, and smaller chunks
-  // instead would drain their queues more often than that saves.
+  // each, max_scatterings + 2 per item) while they take at most 8 GiB and half
+  // of the free memory (ensure_wave): the replay then traces no rays (512x512,
+  // 32 spp, 4 bounces: 10.6 of 38 ms).  The 8 GiB keep the call's memory in
+  // proportion to its other buffers; shorter chunks, whose hits would fit, were
+  // not tried.
   uint64_t const vertices = uint64_t(p->max_scatterings) + 2;
   uint32_t const record = vertices * 36 * chunk <= kHitBytes ? uint32_t(vertices) : 0u;
   WaveState ws{};

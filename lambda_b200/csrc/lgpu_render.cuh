@@ -297,7 +297,7 @@ cudaError_t run_iterations(WaveState& w, uint32_t total, uint32_t max_scatter, c
 // on the device only; blocks past it cost their launch and one read, blocks
 // short of it a loop whose rounds wait for their slowest warp.  A quarter of
 // the queue, but 16 blocks per SM (four rounds of them) at least: against a
-// full grid benchmark frame 270.5 -> 267.9 ms, 4K frame in tiles 33.6 -> 32.6,
+// full grid benchmark frame 270.5 -> 267.9 ms, a 1280x720 frame in tiles 33.6 -> 32.6,
 // 9 instances at 1021x577 8.29 -> 8.12, and a frame whose hits are all of one
 // list 12.14 -> 12.12 ms; 4 blocks per SM at least cost the benchmark frame 276
 // ms, no least number an inverse step 3.88 -> 4.05 ms.  The adjoint's launches

@@ -4,9 +4,14 @@
 // trace_tlas runs one ray to its end; an entered mesh is delimited on the
 // stack by a marker.  The persistent kernels run the same search as a state
 // machine (TraceState) whose node, leaf and object steps the lanes of a warp
-// take together.  Both visit objects and mesh nodes in the order of the
-// nested traversal in lgpu_intersect.cuh, so results are identical to it
-// (and therefore to the reference's intersect::scene, see scene_hit).
+// take together.  Both find the closest hit that the nested traversal in
+// lgpu_intersect.cuh finds, with its rule for ties between objects, but in
+// other trees, with wider box tests (kTravSlack) and in an order that ignores
+// the three low bits of a distance: at an exactly equal distance another face
+// of a mesh can be reported, and a triangle that a ray grazes can be found
+// that the reference's boxes reject.  Rays whose answer depends on the
+// reference's object order among several meshes get the reference's own loop
+// (wf_trace_fallback).
 //
 // The stack keeps its first kSmemStack entries in shared memory, laid out
 // entry-major (entry k of thread t at k*blockDim.x + t) so a warp's pushes

@@ -138,7 +138,6 @@ template <int K, class J>
 __global__ void __launch_bounds__(256) wf_generate_stream(J jobs, WaveState w, DevCounters* cnt) {
   uint32_t const n_new = w.ctl[kCtlNew], first = w.ctl[kCtlFirst], pos = w.ctl[kCtlPos];
   uint32_t paths = 0;
-  uint32_t const cap = w.cap;
   PathBuf const& in = w.in;
   for (uint32_t k = blockIdx.x * blockDim.x + threadIdx.x; k < n_new; k += gridDim.x * blockDim.x) {
     uint32_t const q = first + k;
@@ -385,7 +384,6 @@ __global__ void __launch_bounds__(128, ANY ? 7 : 6) wf_trace_persistent(J jobs, 
   uint32_t tris = 0, insts = 0;
   uint32_t const n = ANY ? w.ctl[kCtlShadow + w.par] : *w.n_in;
   uint32_t* fetch = w.ctl + (ANY ? kCtlSFetch + w.par : uint32_t(kCtlFetch));
-  uint32_t const cap = w.cap;
   unsigned const FULL = 0xFFFFFFFFu;
   int const lane = threadIdx.x & 31;
   TraceState t;
@@ -626,7 +624,7 @@ __device__ __forceinline__ void list_material_groups(const WaveState& w, uint32_
 //     rest), then LGPU_MAT_BLINN, LGPU_MAT_THINFILM and kShadeLamb (Lambertian
 //     and unshaded materials) over their lists, every warp full.
 // The first kind stays for its scenes because a launch more costs them more
-// than full warps give: the 8x8 thumbnail 472 against 508 us with lists, the
+// than full warps give: a 64x64 thumbnail 472 against 508 us with lists, the
 // Lambertian box room 1.85 against 1.90 ms.  The second, against one launch for
 // all but the Blinn and thin-film lists: benchmark frame 277.2 -> 270.2 ms
 // (39.1 ms of shading become 10.8 + 21.5), mixed materials 8.18 -> 7.78 ms.
@@ -894,7 +892,6 @@ __global__ void __launch_bounds__(128) wf_shadow(J jobs, WaveState w, DevCounter
   TravStats ts{0u, 0u, 0u, 0u};
   uint32_t rays = 0;
   uint32_t const n = w.ctl[kCtlShadow + w.par];
-  uint32_t const cap = w.cap;
   for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
     uint32_t const jb = J::kMulti ? w.s_job[i] : 0u;
     const DevScene& S = jobs.scene(jb);
