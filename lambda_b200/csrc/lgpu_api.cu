@@ -519,6 +519,7 @@ int batch_impl(lgpu_ctx* ctx, const lgpu_job* jobs, uint32_t n, float* const* d_
   for (uint32_t k = 0; k < n; k++) {
     DevJob& d = hj[k];
     d.S = ctx->slots[jobs[k].scene].S;
+    table.objects = std::max(table.objects, d.S.n_objects);
     table.mat_types |= d.S.mat_types;
     table.max_bounces = std::max(table.max_bounces, jobs[k].params.max_scatterings);
     d.a = render_args(&jobs[k].params, d.S);

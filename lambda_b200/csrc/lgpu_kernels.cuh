@@ -53,6 +53,7 @@ constexpr int kCtlPos = 13;      //   their first queue position
 constexpr int kCtlListB = 14;    // queue entries that hit a Blinn material
 constexpr int kCtlListT = 15;    //   a thin-film one,
 constexpr int kCtlListL = 16;    //   any other scattering one (shading lists)
+constexpr int kCtlLoopFetch = 17;  // work counter of wf_trace_fallback
 constexpr int kCtlWords = 24;
 constexpr uint32_t kNoShadow = 0xFFFFFFFFu;
 
@@ -239,6 +240,7 @@ struct OneJob {
   RenderArgs a;
   uint32_t npix;
   float* out;
+  uint32_t max_objects() const { return S.n_objects; }
   uint32_t max_scatter() const { return a.max_scatter; }
   bool has_material(int type) const { return (S.mat_types >> type) & 1u; }
   __device__ __forceinline__ const DevScene& scene(uint32_t) const { return S; }
@@ -259,8 +261,10 @@ struct JobTable {
   const uint64_t* item_bases;  // n + 1 entries, the last is the total
   const uint32_t* pix_bases;   // n + 1 entries
   uint32_t n;
+  uint32_t objects;            // of the job's scene that has the most
   uint32_t mat_types;          // of all the jobs' scenes (DevScene::mat_types)
   uint32_t max_bounces;        // of all the jobs (RenderArgs::max_scatter)
+  uint32_t max_objects() const { return objects; }
   uint32_t max_scatter() const { return max_bounces; }
   bool has_material(int type) const { return (mat_types >> type) & 1u; }
   __device__ __forceinline__ const DevScene& scene(uint32_t j) const { return d[j].S; }

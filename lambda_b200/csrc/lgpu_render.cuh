@@ -116,7 +116,7 @@ const WaveOccupancy& wave_occupancy() {
     o.pshadow = blocks_per_sm(wf_trace_persistent<true, K, J>, 128, smem);
     o.gen = blocks_per_sm(wf_generate_stream<K, J>, 256, 0);
     o.fin = blocks_per_sm(wf_finish<K, J>, 256, 0);
-    o.fb = blocks_per_sm(wf_trace_fallback<J>, 128, 0);
+    o.fb = blocks_per_sm(wf_trace_fallback<J>, 128, smem);
     int dev = 0, sms = 0;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
@@ -159,7 +159,7 @@ void launch_closest(const J& jobs, const WaveState& w, const WaveGrids& g, bool 
     wf_trace<J><<<g.trace, 128, kTraceSmem, st>>>(jobs, w, cnt);
   } else {
     wf_trace_persistent<false, K, J><<<g.ptrace, 128, kTraceSmem, st>>>(jobs, w, cnt);
-    wf_trace_fallback<J><<<g.fb, 128, 0, st>>>(jobs, w, cnt);
+    wf_trace_fallback<J><<<g.fb, 128, kTraceSmem, st>>>(jobs, w, jobs.max_objects() <= kMaxLoopObjects, cnt);
   }
 }
 

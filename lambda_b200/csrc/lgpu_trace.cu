@@ -87,7 +87,7 @@ TraceGrids trace_grids(const WaveConfig& cfg) {
     o_shadow = blocks_per_sm(wf_shadow<16, OneJob>, 128, kTraceSmem);
     o_ptrace = blocks_per_sm(wf_trace_persistent<false, 16, OneJob>, 128, kTraceSmem);
     o_pshadow = blocks_per_sm(wf_trace_persistent<true, 16, OneJob>, 128, kTraceSmem);
-    o_fb = blocks_per_sm(wf_trace_fallback<OneJob>, 128, 0);
+    o_fb = blocks_per_sm(wf_trace_fallback<OneJob>, 128, kTraceSmem);
     int dev = 0, n = 0;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev);
@@ -151,7 +151,7 @@ cudaError_t launch_trace_chunk(const DevScene& S, WaveState& w, const float* d_r
       wf_trace<OneJob><<<g.trace, 128, kTraceSmem, st>>>(jobs, w, d_cnt);
     } else {
       wf_trace_persistent<false, 16, OneJob><<<g.ptrace, 128, kTraceSmem, st>>>(jobs, w, d_cnt);
-      wf_trace_fallback<OneJob><<<g.fb, 128, 0, st>>>(jobs, w, d_cnt);
+      wf_trace_fallback<OneJob><<<g.fb, 128, kTraceSmem, st>>>(jobs, w, S.n_objects <= kMaxLoopObjects, d_cnt);
     }
     trace_store<<<(n + 127) / 128, 128, 0, st>>>(S, w, n, d_hits);
   } else {

@@ -61,14 +61,14 @@ struct SplitStack {
   // push and pop branch to a shared or a local access: through at()'s
   // reference the compiler emits generic loads and stores, which cost
   // registers (spills) and issue slots (traversal -6 % measured)
-  __device__ __forceinline__ void push(StackEntry e) {
-    if (sp < kSmemStack) {
-      sm[sp * stride] = e;
+  __device__ __forceinline__ void push(StackEntry e) { put(sp++, e); }
+  __device__ __forceinline__ void put(int k, StackEntry e) {
+    if (k < kSmemStack) {
+      sm[k * stride] = e;
     } else {
       flags |= kTravLocalStack;
-      lm[sp - kSmemStack] = e;
+      lm[k - kSmemStack] = e;
     }
-    sp++;
   }
   __device__ __forceinline__ StackEntry pop() {
     --sp;
@@ -78,6 +78,11 @@ struct SplitStack {
 };
 
 constexpr int kSplitCap = kSmemStack + kLocalStack;
+// Objects of the largest scenes in which wf_trace_fallback may keep the
+// reference's object loop on the stack: its groups and a mesh's entries fit
+// together.
+constexpr uint32_t kMaxLoopObjects = 1024;
+static_assert(kMaxLoopObjects / 32 + kStackCap <= kSplitCap, "object groups and a mesh's entries");
 // push_children (lgpu_intersect.cuh) writing through a SplitStack.  With
 // `sorted` false (any-hit queries, whose boolean answer does not depend on
 // the visiting order) the hit children are pushed in child order.
@@ -322,8 +327,9 @@ __device__ __forceinline__ float min3(float a, float b, float c) {
 }
 
 // Entry distances of all 8 child boxes (node_boxes_t's values, two children
-// per instruction), handed one by one to f(child, entry, hit).
-template <class F>
+// per instruction), handed one by one to f(child, entry, hit).  SLACK: with
+// kTravSlack; without it child_box_t's test.
+template <bool SLACK, class F>
 __device__ __forceinline__ void node_children(const WideNode& nd, const Ray& r, float t_max, F f) {
   bool const nx = r.inv.x < 0.f, ny = r.inv.y < 0.f, nz = r.inv.z < 0.f;
   const ulonglong2* const nrx = reinterpret_cast<const ulonglong2*>(nx ? nd.hix : nd.lox);
@@ -349,9 +355,11 @@ __device__ __forceinline__ void node_children(const WideNode& nd, const Ray& r, 
       unpack2(mul2(add2(k ? d.y : d.x, py), iy), y0, y1);
       unpack2(mul2(add2(k ? g.y : g.x, pz), iz), z0, z1);
       float f0 = fminf(min3(x0, y0, z0), t_max), f1 = fminf(min3(x1, y1, z1), t_max);
-      uint64_t ff;
-      asm("mov.b64 %0, {%1, %2};" : "=l"(ff) : "f"(f0), "f"(f1));
-      unpack2(mul2(ff, slack), f0, f1);
+      if (SLACK) {
+        uint64_t ff;
+        asm("mov.b64 %0, {%1, %2};" : "=l"(ff) : "f"(f0), "f"(f1));
+        unpack2(mul2(ff, slack), f0, f1);
+      }
       f(4 * h + 2 * k, n0, n0 <= f0);
       f(4 * h + 2 * k + 1, n1, n1 <= f1);
     }
@@ -364,7 +372,8 @@ __device__ __forceinline__ void node_children(const WideNode& nd, const Ray& r, 
 // A stack entry is a child reference with its entry distance, or, with
 // kGroupBit set, a node some of whose hit children were not visited yet:
 // their mask in the 8 low bits of t, whose other bits are a lower bound of
-// their entry distances.
+// their entry distances.  In the object loop a group entry in world space is
+// 32 objects from an index on, with the mask of those still to be tested in t.
 constexpr uint32_t kGroupBit = 0x40000000u;  // node indices stay below it (kMaxSlots)
 constexpr uint32_t kNoRef = kEmptyChild;
 
@@ -376,6 +385,12 @@ constexpr uint32_t kLaneTri = 1u << 8;        // tests the triangles of mesh lea
 constexpr uint32_t kLaneObj = 1u << 16;       // tests the object of instance leaf `ref`
 constexpr uint32_t kLaneDone = 1u << 24;      // its ray is finished
 constexpr uint32_t kLaneIdle = (1u << 24) | (1u << 31);  // has no ray (bits 30 and 31 of the sum are not read)
+
+// The three queries of the persistent kernels: closest hits and shadow rays
+// through the instance BVH and the traversal trees, and the reference's loop
+// over the objects in index order through its own trees, with its box tests
+// (no slack) and its order of a node's children.
+constexpr int kQueryClosest = 0, kQueryAny = 1, kQueryLoop = 2;
 
 // trace_tlas as a resumable state machine: trace_begin sets up a ray, then
 // trace_pop and one of trace_node, trace_leaf and trace_object advance it.
@@ -404,8 +419,8 @@ struct TraceState {
   uint32_t ref;    // the node or leaf it does that with
   int base;        // stack height at which the entered mesh is done; -1 in world space
   bool lowered;    // z was lowered for the entered mesh (it loses ties)
-  // 1: closest hit; 2: any hit among the objects below wobj; 3: closest hit
-  // without object wobj (any-hit kernels: 1, any hit without object wobj)
+  // closest hits: 1, closest hit; 2, any hit among the objects below wobj; 3,
+  // closest hit without object wobj (shadow rays: any hit without object wobj)
   int phase;
   uint32_t wobj;
 };
@@ -432,13 +447,13 @@ __device__ __forceinline__ void trace_begin(const DevScene& S, TraceState& t, Sp
 // Takes the next entry from the stack, leaving the entered mesh when its
 // entries are used up.  An entry beyond the closest hit is dropped (the lane
 // pops again).  For a node, `todo` is the mask of the children to test.
-template <bool ANY>
+template <int Q>
 __device__ __forceinline__ void trace_pop(const DevScene& S, TraceState& t, SplitStack& st, uint32_t& todo) {
   if (st.sp <= t.base) {
     // the mesh is done: back to the world ray, and to the distance before it
     // was lowered unless the mesh was hit
     t.base = -1;
-    if (!ANY && t.lowered && t.obj != t.cur) t.z = next_float(t.z);
+    if (Q == kQueryClosest && t.lowered && t.obj != t.cur) t.z = next_float(t.z);
     t.lowered = false;
     t.w.p = f3{st.ws[0], st.ws[128], st.ws[2 * 128]};
     t.w.u = f3{st.ws[3 * 128], st.ws[4 * 128], st.ws[5 * 128]};
@@ -450,13 +465,21 @@ __device__ __forceinline__ void trace_pop(const DevScene& S, TraceState& t, Spli
   }
   StackEntry const e = st.pop();
   uint32_t ref = e.ref;
-  if (ANY) {
+  if (Q == kQueryAny) {
     if (!(ref & kLeafBit) && (ref & kGroupBit)) {
       uint32_t const m = __float_as_uint(e.t);
       uint32_t const c = 31u - __clz(m);
       uint32_t const rest = m ^ (1u << c);
       if (rest) st.push(StackEntry{ref, __uint_as_float(rest)});
       ref = S.nodes[ref ^ kGroupBit].child[c];
+    }
+  } else if (Q == kQueryLoop) {
+    if (t.base < 0) {
+      uint32_t const m = __float_as_uint(e.t), rest = m & (m - 1u);
+      if (rest) st.push(StackEntry{ref, __uint_as_float(rest)});
+      ref = kLeafBit | ((ref ^ kGroupBit) + uint32_t(__ffs(m) - 1));
+    } else if (e.t > t.z) {
+      return;
     }
   } else {
     uint32_t bound = __float_as_uint(e.t);
@@ -485,19 +508,43 @@ __device__ __forceinline__ void trace_pop(const DevScene& S, TraceState& t, Spli
 // min/max operations where a sorting network takes 38 and up to 8 pushes.
 // Shadow rays visit them from the last to the first (their answer does not
 // depend on the order, and distance order is slower), as one group.
-template <bool ANY>
+// The object loop pushes them all, as push_children does, but the nearest.
+template <int Q>
 __device__ __forceinline__ void trace_node(const DevScene& S, TraceState& t, SplitStack& st, uint32_t todo) {
   uint32_t const ref = t.ref;
   uint32_t next = kNoRef;
   const WideNode& nd = S.nodes[ref];
+  if (Q == kQueryLoop) {
+    float tc[8];
+    int hits = 0, rank[8];
+    node_children<false>(nd, t.w, t.z, [&](int c, float entry, bool hit) {
+      tc[c] = hit ? entry : 0.f;
+      hits += hit ? 1 : 0;
+    });
+    if (st.sp + hits > kSplitCap) {
+      st.flags |= kTravOverflow;
+      t.kind = kLaneDone;
+      return;
+    }
+    child_ranks(tc, rank);
+#pragma unroll
+    for (int c = 0; c < 8; c++)
+      if (tc[c] != 0.f) {
+        if (rank[c] == hits - 1) next = nd.child[c];
+        else st.put(st.sp + rank[c], StackEntry{nd.child[c], tc[c]});
+      }
+    st.sp += hits > 0 ? hits - 1 : 0;
+    trace_next(t, next);
+    return;
+  }
   if (st.sp + 2 > kSplitCap) {
     st.flags |= kTravOverflow;
     t.kind = kLaneDone;
     return;
   }
   uint32_t m = 0;
-  if (ANY) {
-    node_children(nd, t.w, t.z, [&](int c, float, bool hit) {
+  if (Q == kQueryAny) {
+    node_children<true>(nd, t.w, t.z, [&](int c, float, bool hit) {
       if (hit) m |= 1u << c;
     });
     if (m) {
@@ -510,7 +557,7 @@ __device__ __forceinline__ void trace_node(const DevScene& S, TraceState& t, Spl
     return;
   }
   uint32_t key[8];
-  node_children(nd, t.w, t.z, [&](int c, float tc, bool hit) {
+  node_children<true>(nd, t.w, t.z, [&](int c, float tc, bool hit) {
     key[c] = hit ? ((__float_as_uint(tc) & ~7u) | uint32_t(7 - c)) : 0xFFFFFFFFu;
     if (hit) m |= 1u << c;
   });
@@ -552,9 +599,9 @@ __device__ __forceinline__ void trace_node(const DevScene& S, TraceState& t, Spl
 
 // Tests the triangles of mesh leaf t.ref.  accept(face, b0, b1, b2, point,
 // distance) records a closer hit.
-template <bool ANY, class A>
+template <int Q, class A>
 __device__ __forceinline__ void trace_leaf(const DevScene& S, TraceState& t, uint32_t& tris, A accept) {
-  bool const any = ANY || t.phase == 2;
+  bool const any = Q == kQueryAny || (Q == kQueryClosest && t.phase == 2);
   uint32_t const cnt = ((t.ref >> 28) & 7u) + 1u;
   uint32_t const slot = t.ref & kSlotMask;
   t.kind = kLanePop;
@@ -579,15 +626,15 @@ __device__ __forceinline__ void trace_leaf(const DevScene& S, TraceState& t, uin
 // Tests the object of instance leaf t.ref (the rest of the leaf waits on the
 // stack): a sphere or plane in full, a mesh by its bounds, after which the
 // next step enters its tree.
-template <bool ANY, class A>
+template <int Q, class A>
 __device__ __forceinline__ void trace_object(const DevScene& S, TraceState& t, SplitStack& st, uint32_t& insts,
                                              A accept) {
-  bool const any = ANY || t.phase == 2;
+  bool const any = Q == kQueryAny || (Q == kQueryClosest && t.phase == 2);
   uint32_t const cnt = ((t.ref >> 28) & 7u) + 1u;
   uint32_t const slot = t.ref & kSlotMask;
   t.kind = kLanePop;
-  uint32_t const i = S.tlas_objects[slot];
-  if (cnt > 1) {
+  uint32_t const i = Q == kQueryLoop ? slot : S.tlas_objects[slot];
+  if (Q != kQueryLoop && cnt > 1) {
     if (st.sp + 1 > kSplitCap) {
       st.flags |= kTravOverflow;
       t.kind = kLaneDone;
@@ -595,10 +642,11 @@ __device__ __forceinline__ void trace_object(const DevScene& S, TraceState& t, S
     }
     st.push(StackEntry{kLeafBit | ((cnt - 2u) << 28) | (slot + 1u), 0.f});
   }
-  if (ANY ? i == t.wobj : ((t.phase == 2 && i >= t.wobj) || (t.phase == 3 && i == t.wobj))) return;
+  if (Q == kQueryAny && i == t.wobj) return;
+  if (Q == kQueryClosest && ((t.phase == 2 && i >= t.wobj) || (t.phase == 3 && i == t.wobj))) return;
   insts++;
   const DevObject& ob = S.objects[i];
-  bool const low = !any && t.obj != UINT32_MAX && i < t.obj;
+  bool const low = Q == kQueryClosest && !any && t.obj != UINT32_MAX && i < t.obj;
   // a lower-index object loses ties: it has to be hit below the next float
   float const z = low ? prev_float(t.z) : t.z;
   Ray const li = to_local(ob, t.w);
@@ -628,10 +676,12 @@ __device__ __forceinline__ void trace_object(const DevScene& S, TraceState& t, S
   bool inside;
   float ex;
   float r0 = aabb_scalar(m.bounds, li, z, inside, ex);
-  if (!ANY && r0 != kFltMax && inside) t.n_inside++;
-  // only shadow rays (and the reference's loop) enter a mesh from inside at
-  // its exit distance
-  if (!ANY && r0 != kFltMax && inside) r0 = kBias;
+  // shadow rays and the reference's loop enter a mesh from inside at its exit
+  // distance
+  if (Q == kQueryClosest && r0 != kFltMax && inside) {
+    t.n_inside++;
+    r0 = kBias;
+  }
   if (r0 == kFltMax || r0 > z) return;
   st.ws[0] = t.w.p.x;
   st.ws[128] = t.w.p.y;
@@ -648,7 +698,7 @@ __device__ __forceinline__ void trace_object(const DevScene& S, TraceState& t, S
   t.cur_exit = inside ? ex : -1.f;
   t.lowered = low;
   t.base = st.sp;
-  trace_next(t, m.trav_root);
+  trace_next(t, Q == kQueryLoop ? m.root : m.trav_root);
 }
 
 // intersect::scene for the wavefront kernels: the instance BVH through

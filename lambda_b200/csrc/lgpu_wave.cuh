@@ -123,6 +123,7 @@ __global__ void wf_plan(WaveState w, uint32_t total) {
   w.ctl[kCtlFetch] = 0;
   w.ctl[kCtlSFetch + w.par] = 0;
   w.ctl[kCtlFallback] = 0;
+  w.ctl[kCtlLoopFetch] = 0;
   w.ctl[kCtlEnded + w.par] = 0;
   w.ctl[kCtlListB] = 0;
   w.ctl[kCtlListT] = 0;
@@ -375,6 +376,7 @@ constexpr uint32_t kMinShare = 8;
 // queries (5: +9 %, 7: +1 %).
 template <bool ANY, int K, class J>
 __global__ void __launch_bounds__(128, ANY ? 7 : 6) wf_trace_persistent(J jobs, WaveState w, DevCounters* cnt) {
+  constexpr int Q = ANY ? kQueryAny : kQueryClosest;
   extern __shared__ StackEntry smem_stack[];
   StackEntry lm[kLocalStack];
   SplitStack st{smem_stack + threadIdx.x, blockDim.x, lm, 0, 0u};
@@ -421,8 +423,8 @@ __global__ void __launch_bounds__(128, ANY ? 7 : 6) wf_trace_persistent(J jobs, 
           // others, and the reference's loop answers (wf_trace_fallback).
           //
           // Asking first in that case too would leave 1 in 50 to 120 of those
-          // rays for the loop (box room 1.86 instead of 2.08 ms, 14 box rooms
-          // with instances 8.9 instead of 11.3 ms), but gives other answers:
+          // rays for the loop (box room 1.86 instead of 1.91 ms, 14 box rooms
+          // with instances 8.9 instead of 10.5 ms), but gives other answers:
           // the loop's exact box tests in the reference's trees reject
           // triangles that a ray grazes and that this search finds (one batch
           // in 75 of such rooms had a different image).
@@ -480,54 +482,151 @@ __global__ void __launch_bounds__(128, ANY ? 7 : 6) wf_trace_persistent(J jobs, 
     }
     const DevScene& S = jobs.scene(jb);
     uint32_t todo = 0xFFu;
-    if (t.kind == kLanePop) trace_pop<ANY>(S, t, st, todo);
+    if (t.kind == kLanePop) trace_pop<Q>(S, t, st, todo);
     int const n_node = __popc(__ballot_sync(FULL, t.kind == kLaneNode));
     nodes += n_node;
-    if (t.kind == kLaneNode) trace_node<ANY>(S, t, st, todo);
-    if ((n_tri >= kTriLanes || n_tri >= n_node) && t.kind == kLaneTri) trace_leaf<ANY>(S, t, tris, accept);
-    if ((n_obj >= kObjLanes || n_obj >= n_node) && t.kind == kLaneObj) trace_object<ANY>(S, t, st, insts, accept);
+    if (t.kind == kLaneNode) trace_node<Q>(S, t, st, todo);
+    if ((n_tri >= kTriLanes || n_tri >= n_node) && t.kind == kLaneTri) trace_leaf<Q>(S, t, tris, accept);
+    if ((n_obj >= kObjLanes || n_obj >= n_node) && t.kind == kLaneObj) trace_object<Q>(S, t, st, insts, accept);
   }
   TravStats const ts{st.flags, lane == 0 ? nodes : 0u, tris, insts};
   flush_counters(cnt, lane == 0 ? rays : 0u, 0u, ts, 0u);
 }
 
 // Extension rays whose closest hit depends on the reference's object order
-// (see scene_hit): the linear object loop, one warp per ray.  The lanes
-// first test 32 objects at a time with an unbounded distance (the objects
-// the ray cannot hit at all drop out); lane 0 then runs the reference's
-// loop over the remaining ones in index order.  A launch has few such rays
-// (about ten), so its time is the latency of one ray's loop, which the
-// filter shortens from every object to the handful the ray can reach.
+// (see scene_hit): the reference's loop over the objects, in its trees, with
+// its tests and its order.  The objects that a ray cannot hit at any distance
+// drop out first, 32 at a time by all lanes of a warp (every test of the loop
+// only gets stricter as the distance bound shrinks).
+//
+// Few rays, whose time is the latency of one ray's loop: one warp per ray,
+// whose first lane runs the loop over the remaining objects.  From kManyLoop
+// rays on, the steps of wf_trace_persistent with the loop's tests (kQueryLoop),
+// shared by the lanes whatever object each ray is at; the remaining objects
+// wait on the stack of the ray's lane, the lowest indices on top, which holds
+// those of kMaxLoopObjects objects (`steps`: no scene has more).
+// Ray queries, closest-hit kernel included: 144,091 such rays among 40
+// overlapping objects 5.4 ms with a warp per ray, 2.8 with steps; 116,177 among
+// 1,000 objects 8.0, 5.5; 9,458 among 40 0.80, 0.75; 4,239 among 150 0.455,
+// 0.469.  Box room 256x256, 16 spp (90,378 in 10 launches) 2.34, 2.18 ms; 64x64,
+// 4 spp (1,490) 0.806, 0.846.  As a phase of the closest-hit kernel the steps
+// spilled registers there (benchmark frame +3.5 %).
+constexpr uint32_t kManyLoop = 8192;
+
 template <class J>
-__global__ void __launch_bounds__(128) wf_trace_fallback(J jobs, WaveState w, DevCounters* cnt) {
-  StackEntry lstack[kStackCap];
-  TravStats ts{0u, 0u, 0u, 0u};
+__global__ void __launch_bounds__(128, 6) wf_trace_fallback(J jobs, WaveState w, bool steps, DevCounters* cnt) {
+  extern __shared__ StackEntry smem_stack[];
+  StackEntry lm[kLocalStack];
+  static_assert(kLocalStack >= kStackCap, "a mesh's entries");
   uint32_t const n = w.ctl[kCtlFallback];
-  uint32_t const lane = threadIdx.x & 31u;
-  uint32_t const nwarps = (gridDim.x * blockDim.x) >> 5;
-  for (uint32_t i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; i < n; i += nwarps) {
-    uint32_t const p = w.fb_queue[i];
-    const DevScene& S = jobs.scene(J::kMulti ? w.in.job[p] : 0u);
-    Ray const r = load_ray(w.in.ra, w.in.rb, p);
-    HitRec h;
-    clear_hit(h, kFltMax);
-    h.inside = false;
-    for (uint32_t base = 0; base < S.n_objects; base += 32) {
-      uint32_t const o = base + lane;
-      unsigned m = __ballot_sync(0xFFFFFFFFu, o < S.n_objects && object_may_hit(S, o, r));
-      if (lane == 0)
-        while (m) {
-          uint32_t const b = uint32_t(__ffs(m) - 1);
-          m &= m - 1u;
-          object_hit<false>(S, base + b, r, h, lstack, ts, kRefOrder);
-        }
-      __syncwarp();
+  unsigned const FULL = 0xFFFFFFFFu;
+  int const lane = threadIdx.x & 31;
+  uint32_t const warps = gridDim.x * (blockDim.x >> 5);
+  if (n < kManyLoop || !steps) {
+    TravStats ts{0u, 0u, 0u, 0u};
+    for (uint32_t i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; i < n; i += warps) {
+      uint32_t const p = w.fb_queue[i];
+      const DevScene& S = jobs.scene(J::kMulti ? w.in.job[p] : 0u);
+      Ray const r = load_ray(w.in.ra, w.in.rb, p);
+      HitRec h;
+      clear_hit(h, kFltMax);
+      h.inside = false;
+      for (uint32_t base = 0; base < S.n_objects; base += 32) {
+        uint32_t const o = base + uint32_t(lane);
+        unsigned m = __ballot_sync(FULL, o < S.n_objects && object_may_hit(S, o, r));
+        if (lane == 0)
+          while (m) {
+            uint32_t const b = uint32_t(__ffs(m) - 1);
+            m &= m - 1u;
+            object_hit<false>(S, base + b, r, h, lm, ts, kRefOrder);
+          }
+        __syncwarp();
+      }
+      if (lane == 0) {
+        store_hit(w, p, h);
+        atomicAdd(&cnt->ordered, 1ull);
+      }
     }
-    if (lane == 0) {
-      store_hit(w, p, h);
-      atomicAdd(&cnt->ordered, 1ull);
-    }
+    flush_counters(cnt, 0u, 0u, ts, 0u);
+    return;
   }
+  SplitStack st{smem_stack + threadIdx.x, blockDim.x, lm, 0, 0u};
+  __shared__ float wsave[9 * 128];  // launched with 128 threads
+  st.ws = wsave + threadIdx.x;
+  uint32_t rays = 0, nodes = 0;  // of the warp
+  uint32_t tris = 0, insts = 0;
+  TraceState t;
+  t.kind = kLaneIdle;
+  int wait = kRefill;
+  // (32 except where n is below the number of lanes)
+  uint32_t const share = min(32u, (n + warps - 1u) / warps);
+  bool const on = uint32_t(lane) < share;
+  uint32_t idx = 0, jb = 0;
+  auto accept = [&](uint32_t face, float b0, float b1, float b2, f3 pl, float z) {
+    store_hit_point(w, idx, face, b0, b1, b2, pl, z);
+  };
+  while (true) {
+    uint32_t const sum = __reduce_add_sync(FULL, t.kind);
+    int const n_tri = int((sum >> 8) & 0xFFu), n_obj = int((sum >> 16) & 0xFFu);
+    if (int((sum >> 24) & 0x3Fu) >= wait) {
+      if (t.kind == kLaneDone) {
+        t.kind = kLaneIdle;
+        w.hobj[idx] = t.obj;
+      }
+      unsigned idle = __ballot_sync(FULL, t.kind == kLaneIdle && on);
+      if (wait == kRefill && idle) {
+        uint32_t const want = uint32_t(__popc(idle));
+        int const leader = __ffs(idle) - 1;
+        uint32_t base = 0;
+        if (lane == leader) base = atomicAdd(w.ctl + kCtlLoopFetch, want);
+        base = __shfl_sync(FULL, base, leader);
+        uint32_t const got = min(base < n ? n - base : 0u, want);
+        uint32_t const k = uint32_t(__popc(idle & ((1u << lane) - 1u)));
+        bool const fresh = t.kind == kLaneIdle && on && k < got;
+        if (fresh) {
+          idx = w.fb_queue[base + k];
+          if (J::kMulti) jb = w.in.job[idx];
+          t.w = load_ray(w.in.ra, w.in.rb, idx);
+          t.z = kFltMax;
+          t.obj = UINT32_MAX;
+          t.base = -1;
+          t.kind = kLanePop;
+          st.sp = 0;
+        }
+        for (unsigned m = __ballot_sync(FULL, fresh); m; m &= m - 1u) {
+          int const src = __ffs(m) - 1;
+          const DevScene& S = jobs.scene(__shfl_sync(FULL, jb, src));
+          Ray r;
+          r.p = f3{__shfl_sync(FULL, t.w.p.x, src), __shfl_sync(FULL, t.w.p.y, src), __shfl_sync(FULL, t.w.p.z, src)};
+          r.u = f3{__shfl_sync(FULL, t.w.u.x, src), __shfl_sync(FULL, t.w.u.y, src), __shfl_sync(FULL, t.w.u.z, src)};
+          r.inv = f3{0.f, 0.f, 0.f};  // the tests below use the local rays' own
+          for (uint32_t b = (S.n_objects + 31u) / 32u; b-- > 0u;) {
+            uint32_t const o = 32u * b + uint32_t(lane);
+            unsigned const may = __ballot_sync(FULL, o < S.n_objects && object_may_hit(S, o, r));
+            if (lane == src && may) st.push(StackEntry{kGroupBit | (32u * b), __uint_as_float(may)});
+          }
+        }
+        rays += got;
+        if (base + want >= n || share < 32u) wait = 0;
+      }
+      idle = __ballot_sync(FULL, t.kind == kLaneIdle);
+      if (wait != kRefill) {
+        if (idle == FULL) break;
+        wait = __popc(idle) + 1;
+      }
+      continue;
+    }
+    const DevScene& S = jobs.scene(jb);
+    uint32_t todo = 0;
+    if (t.kind == kLanePop) trace_pop<kQueryLoop>(S, t, st, todo);
+    int const n_node = __popc(__ballot_sync(FULL, t.kind == kLaneNode));
+    nodes += n_node;
+    if (t.kind == kLaneNode) trace_node<kQueryLoop>(S, t, st, todo);
+    if ((n_tri >= kTriLanes || n_tri >= n_node) && t.kind == kLaneTri) trace_leaf<kQueryLoop>(S, t, tris, accept);
+    if ((n_obj >= kObjLanes || n_obj >= n_node) && t.kind == kLaneObj) trace_object<kQueryLoop>(S, t, st, insts, accept);
+  }
+  if (lane == 0 && rays) atomicAdd(&cnt->ordered, static_cast<unsigned long long>(rays));
+  TravStats const ts{st.flags, lane == 0 ? nodes : 0u, tris, insts};
   flush_counters(cnt, 0u, 0u, ts, 0u);
 }
 

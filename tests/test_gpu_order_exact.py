@@ -70,9 +70,10 @@ def edge_rays(corners, n, seed):
     return np.concatenate([o, d.astype(np.float32)], axis=1)
 
 
-# 6 and 40 objects: one and two groups of 32 in the object loop; 1025: many, and
-# meshes that several objects share, so that equal distances tie
-@pytest.mark.parametrize("n_objects,n_meshes,per_mesh", [(6, 6, 6), (40, 40, 2), (1025, 8, 6)])
+# 6 and 40 objects: one and two groups of 32 in the object loop; 1024 and 1025:
+# its largest scene in steps, and the smallest that always has a warp per ray,
+# with meshes that several objects share, so that equal distances tie
+@pytest.mark.parametrize("n_objects,n_meshes,per_mesh", [(6, 6, 6), (40, 40, 2), (1024, 8, 6), (1025, 8, 6)])
 def test_equals_the_reference_order(n_objects, n_meshes, per_mesh):
     from lambda_b200.renderer import Context
     from lambda_b200.scene import FlatScene
@@ -92,3 +93,30 @@ def test_equals_the_reference_order(n_objects, n_meshes, per_mesh):
                          (a["face"] != b["face"]))
     assert bad.size == 0, (bad.size, a[bad[:3]], b[bad[:3]])
     assert a.tobytes() == b.tobytes()
+
+
+@pytest.mark.parametrize("n_objects,n_meshes,per_mesh", [(6, 6, 6), (40, 40, 2)])
+def test_few_and_many_rays(n_objects, n_meshes, per_mesh):
+    """Launches of few order-dependent rays (a warp each) and of 8192 and more
+    (in steps): on both sides of the line, with single lanes and full warps."""
+    from lambda_b200.renderer import Context
+    from lambda_b200.scene import FlatScene
+    sc, corners = scene_of(n_objects, n_meshes, per_mesh, n_objects)
+    ctx = Context(0)
+    ctx.upload(FlatScene(sc))
+    rays = edge_rays(corners, 60_000, 4)
+    b = ctx.trace(rays, flags=L.FLAG_REFERENCE_ORDER)
+    ends = [1, 2, 33, 1000]
+    for want in (8191, 8192, 8193, 14207, 14208):
+        lo, hi = 0, len(rays)  # the number of order-dependent rays grows with the number of rays
+        while lo < hi:
+            m = (lo + hi) // 2
+            ctx.trace(rays[:m])
+            lo, hi = (m + 1, hi) if ctx.stats()["order_rays"] < want else (lo, m)
+        ctx.trace(rays[:lo])
+        assert ctx.stats()["order_rays"] == want
+        ends.append(lo)
+    for n in ends + [len(rays)]:
+        a = ctx.trace(rays[:n])
+        assert a.tobytes() == b[:n].tobytes(), n
+    ctx.close()
