@@ -202,8 +202,8 @@ static_assert(kMaxWhole <= WaveLaunch::kSlots && kMaxWhole % 2 == 0, "iterations
 // pair, the next while the last one's queue length comes back, until that is 0
 // or all are enqueued.  (Iterations after the paths have ended cost 25 us each:
 // enqueued all at once and unasked, a view of nothing with 14 scatterings took
-// 511 instead of 197 us, 8x8 pixels with p = 0.3 663 instead of 421; asking
-// costs a thumbnail of 6 iterations 491 -> 498 us.)
+// 511 instead of 141 us, 8x8 pixels with p = 0.3 663 instead of 416; asking
+// costs a thumbnail of 6 iterations 484 -> 499 us.)
 // Otherwise the counters are read back every kItersPerCheck iterations; with
 // a graph cache and no per-kernel timing, those after the first are captured
 // as a CUDA graph while the device runs the first ones (a capture costs the
@@ -227,18 +227,21 @@ cudaError_t run_iterations(WaveState& w, uint32_t total, uint32_t max_scatter, c
     cudaMemcpyAsync(ws.h_ctl, ws.ctl, ctl_bytes, cudaMemcpyDeviceToHost, st);
   };
   if (whole) {
+    auto ask = [&](uint32_t k) {
+      cudaMemcpyAsync(w.h_ctl + kCtlWords + k, w.n_in, sizeof(uint32_t), cudaMemcpyDeviceToHost, st);
+      cudaEventRecord(run->asked[k], st);
+    };
     for (uint32_t it = 0; it < max_scatter + 2; it += 2) {
+      // this pair's queue length decides on the pair after the next, and the
+      // first iteration's on the second pair
       uint32_t const k = (it / 2) & 1u, left = max_scatter + 2 - it;
       for (uint32_t j = 0; j < 2; j++) {
         issue(w, it + j == 0);
         swap_queues(w);
+        if (it + j == 0 && left > 2) ask(1);
       }
-      // this pair's queue length decides on the pair after the next
-      if (left > 4) {
-        cudaMemcpyAsync(w.h_ctl + kCtlWords + k, w.n_in, sizeof(uint32_t), cudaMemcpyDeviceToHost, st);
-        cudaEventRecord(run->asked[k], st);
-      }
-      if (it == 0 || left <= 2) continue;
+      if (left > 4) ask(k);
+      if (left <= 2) continue;
       cudaError_t const e = cudaEventSynchronize(run->asked[k ^ 1u]);
       if (e != cudaSuccess) return e;
       if (w.h_ctl[kCtlWords + (k ^ 1u)] == 0) break;
